@@ -91,10 +91,11 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
     headers = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [ROOT / "include" / "tgo_mmq.h",
                                                                       BUILD / "iq2s_grid.inc"]
     jobs = []
-    for qt in QUANT_TYPES:
-        jobs.append((CSRC / "mmq_inst.cu", BUILD / f"mmq_inst_{qt}.o", [f"-DTGO_QT={qt}"]))
+    for src in sorted(CSRC.glob("*_inst.cu")):   # one object per quant type
+        for qt in QUANT_TYPES:
+            jobs.append((src, BUILD / f"{src.stem}_{qt}.o", [f"-DTGO_QT={qt}"]))
     for src in sorted(CSRC.glob("*.cu")):
-        if src.name != "mmq_inst.cu":
+        if not src.stem.endswith("_inst"):
             jobs.append((src, BUILD / (src.stem + ".o"), []))
     todo = [(s, o, f) for (s, o, f) in jobs if force or not _newer(o, [s, *headers])]
 

@@ -18,6 +18,7 @@
 #include <cudaTypedefs.h>
 
 #include "mmq_launch.h"
+#include "mmq_small_launch.h"
 
 namespace tgo {
 
@@ -445,8 +446,8 @@ static int plan_split(int64_t rows, int64_t N, int64_t K, int64_t tile_m, int64_
 
 struct Problem {
     const void* act[2];
-    const void* wgt[2];
-    void* out[2];
+    const void* wgt[kSmallMaxSets];   // more than two: few-token kernel only
+    void* out[kSmallMaxSets];
     int nsets;
     int64_t rows, N, K, E;
     int qt, mode;
@@ -484,6 +485,119 @@ static int check_common(const Problem& p) {
     return TGO_OK;
 }
 
+// ------------------------------------------------------------------ few tokens per weight row
+static int small_smem(int qt, int nkb, int nt, int kw, int rw, int stages, int groups) {
+    switch (qt) {
+        case QT_Q3_K: return small_smem_11(nkb, nt, kw, rw, stages, groups);
+        case QT_Q4_K: return small_smem_12(nkb, nt, kw, rw, stages, groups);
+        case QT_Q5_K: return small_smem_13(nkb, nt, kw, rw, stages, groups);
+        case QT_Q6_K: return small_smem_14(nkb, nt, kw, rw, stages, groups);
+        default: return small_smem_22(nkb, nt, kw, rw, stages, groups);
+    }
+}
+static int launch_small(int qt, int nt, const SmallArgs& args, int grid, int smem, cudaStream_t stream) {
+    switch (qt) {
+        case QT_Q3_K: return launch_small_11(nt, args, grid, smem, stream);
+        case QT_Q4_K: return launch_small_12(nt, args, grid, smem, stream);
+        case QT_Q5_K: return launch_small_13(nt, args, grid, smem, stream);
+        case QT_Q6_K: return launch_small_14(nt, args, grid, smem, stream);
+        default: return launch_small_22(nt, args, grid, smem, stream);
+    }
+}
+
+constexpr int64_t kSmallRounds = 3;     // row tiles per warp from which on the reduction is not sliced
+// Most rows per group for which the few-token kernel is the faster one.  Its time grows with the
+// tokens (every 8 are one more mma per fragment), the GEMM's hardly does below 256.  Dense: measured
+// on 248320 x 2048 at 24 rows 129-181 us against 155-244 us for the five types; what follows up to 32
+// would win less and less.  Grouped, 256 experts, skewed counts (a mean of m comes with groups of 3 m,
+// which take several tiles): the times cross between a mean of 12 (Q6_K) and 22 (Q3_K, IQ2_S, whose
+// decode costs the GEMM most).
+static int64_t small_max_mean(int qt, bool grouped) {
+    if (!grouped) return 24;
+    switch (qt) {
+        case QT_Q3_K: case QT_IQ2_S: return 20;
+        case QT_Q6_K: return 12;
+        default: return 13;
+    }
+}
+// groups of 8 tokens per tile for a mean of `mean` rows per group
+static int small_tile_groups(int64_t mean) {
+    const int64_t nt = (mean * 5 / 4 + 7) / 8;
+    return static_cast<int>(nt < 1 ? 1 : nt > 4 ? 4 : nt);
+}
+// Whether the few-token kernel (mmq_small.cuh) takes this forward product, and its launch shape.
+struct SmallPlan {
+    int nt, kw, rw, stages, smem, grid;
+};
+static bool plan_small(const Problem& p, SmallPlan& s) {
+    if (p.mode != kFwd || wide_tiles_env() >= 0 || wanted_cta_group() == 1) return false;   // the GEMM's variants asked for by name
+    const int64_t groups = p.experts != nullptr ? p.groups : 1;
+    if (groups > kSmallMaxGroups || p.rows > groups * small_max_mean(p.qt, p.experts != nullptr)) return false;
+    const int64_t mean = (p.rows + groups - 1) / groups;
+    const int nkb = static_cast<int>(p.K / 256);
+    s.nt = p.experts == nullptr ? static_cast<int>((mean + 7) / 8) : small_tile_groups(mean);
+    // Reduction slices: none where the row tiles alone keep every warp busy for a few rounds (a slice
+    // costs a barrier and a pass through shared memory per tile), up to one block per warp where
+    // they do not even cover the SMs.
+    const int64_t tiles = p.experts == nullptr ? 1 : (p.rows < groups ? p.rows : groups);   // about; the device knows
+    const int64_t row_tiles = tiles * p.nsets * ((p.N + 15) / 16);
+    const int64_t warps = static_cast<int64_t>(num_sms()) * kSmallWarps;
+    int64_t kw = row_tiles > 0 ? (kSmallRounds * warps + row_tiles - 1) / row_tiles : kSmallWarps;
+    if (kw > nkb) kw = nkb;
+    if (kw > kSmallWarps) kw = kSmallWarps;
+    const int64_t rounds = (nkb + kw - 1) / kw;
+    s.kw = static_cast<int>((nkb + rounds - 1) / rounds);   // the fewest slices with that many blocks at most
+    int64_t rw = kSmallWarps / s.kw;
+    if (rw > row_tiles / num_sms()) rw = row_tiles / num_sms();
+    if (rw < 1) rw = 1;
+    const int lists = p.experts != nullptr ? static_cast<int>(groups) : 0;
+    for (;; --rw) {
+        if (rw < 1) return false;   // the fragments of x alone do not fit
+        s.rw = static_cast<int>(rw);
+        for (s.stages = 4; s.stages >= 2; --s.stages) {
+            s.smem = small_smem(p.qt, nkb, s.nt, s.kw, s.rw, s.stages, lists);
+            if (s.smem <= kSmallSmemLimit) break;
+        }
+        if (s.stages >= 2) break;
+    }
+    int per_sm = kSmallWarps / (s.kw * s.rw);                 // 128 registers a thread
+    const int fit = kSmallSmemLimit / (s.smem + 1024);
+    if (per_sm > fit) per_sm = fit > 0 ? fit : 1;
+    const int64_t most = (p.experts == nullptr ? 1 : p.rows / (8 * s.nt) + groups) * p.nsets * ((p.N + 16 * s.rw - 1) / (16 * s.rw));
+    if (most > INT32_MAX / 2) return false;
+    const int64_t slots = static_cast<int64_t>(num_sms()) * per_sm;
+    s.grid = static_cast<int>(most < slots ? most : slots);
+    return true;
+}
+
+static int run_small(const Problem& p, const SmallPlan& s, cudaStream_t stream) {
+    SmallArgs a;
+    memset(&a, 0, sizeof(a));
+    for (int i = 0; i < p.nsets; ++i) {
+        a.wgt[i] = static_cast<const uint8_t*>(p.wgt[i]);
+        a.out[i] = static_cast<__nv_bfloat16*>(p.out[i]);
+    }
+    a.act = static_cast<const __nv_bfloat16*>(p.act[0]);
+    a.experts = p.experts;
+    a.offsets = p.offsets;
+    a.out_rows = reinterpret_cast<__nv_bfloat16* const*>(p.out_rows);
+    a.iq2s_grid = grid_ptr();
+    if (a.iq2s_grid == nullptr) return fail(TGO_E_CUDA, "cudaGetSymbolAddress failed");
+    a.tile_count = p.experts != nullptr ? static_cast<int*>(p.ws) : nullptr;
+    a.row_bytes = static_cast<int>((p.K / 256) * tgo_block_bytes(p.qt));
+    a.wgt_bytes = p.E * p.N * a.row_bytes;
+    a.rows = static_cast<int>(p.rows);
+    a.out_features = static_cast<int>(p.N);
+    a.in_features = static_cast<int>(p.K);
+    a.nsets = p.nsets;
+    a.groups = p.experts != nullptr ? static_cast<int>(p.groups) : 0;
+    a.num_experts = static_cast<int>(p.E);
+    a.kw = s.kw; a.rw = s.rw; a.stages = s.stages;
+    const int e = launch_small(p.qt, s.nt, a, s.grid, s.smem, stream);
+    if (e != 0) return cuda_fail(static_cast<cudaError_t>(e), "mmq_small_kernel launch");
+    return check_status_if_asked(stream);
+}
+
 static int run_problem(const Problem& p, cudaStream_t stream) {
     int rc = check_common(p);
     if (rc != TGO_OK) return rc;
@@ -493,6 +607,9 @@ static int run_problem(const Problem& p, cudaStream_t stream) {
             return fail(TGO_E_WORKSPACE, "workspace has %lld bytes, need %lld", (long long)p.ws_bytes, (long long)need);
         if (!aligned16(p.ws)) return fail(TGO_E_ARG, "workspace pointer must be 16-byte aligned");
     }
+    if (p.E * p.N > INT32_MAX) return fail(TGO_E_ARG, "experts * out_features exceeds the kernel limit of 2^31-1");
+    SmallPlan small;
+    if (plan_small(p, small)) return run_small(p, small, stream);
     GemmArgs a;
     memset(&a, 0, sizeof(a));
     const int64_t red = p.mode == kFwd ? p.K : p.N;  // activation row length
@@ -508,7 +625,6 @@ static int run_problem(const Problem& p, cudaStream_t stream) {
         a.out[s] = static_cast<__nv_bfloat16*>(p.out[(p.mode == kFwd && s < p.nsets) ? s : 0]);
     }
     const int64_t bb = tgo_block_bytes(p.qt);
-    if (p.E * p.N > INT32_MAX) return fail(TGO_E_ARG, "experts * out_features exceeds the kernel limit of 2^31-1");
     for (int s = 0; s < p.nsets; ++s) {
         rc = make_wgt_maps(a.wgt_maps[s], p.wgt[s], p.E * p.N, (p.K / 256) * bb, copy_bytes_of(p.qt),
                            p.mode == kFwd ? 128 : 64, a.wgt_classes, a.wgt_classes_log2);
@@ -749,6 +865,14 @@ int tgo_mmq_fwd_multi(const void* x, const void* const* packed_weights, void* co
                       int64_t out_features, int64_t in_features, int quant_type, void* stream) {
     if (packed_weights == nullptr || ys == nullptr) return fail(TGO_E_ARG, "null pointer array");
     if (num_weights < 1 || num_weights > 4) return fail(TGO_E_ARG, "num_weights must be in 1..4; got %lld", (long long)num_weights);
+    Problem all = {};
+    all.nsets = static_cast<int>(num_weights);
+    all.act[0] = x;
+    for (int i = 0; i < all.nsets; ++i) { all.wgt[i] = packed_weights[i]; all.out[i] = ys[i]; }
+    all.rows = rows; all.N = out_features; all.K = in_features; all.E = 1; all.qt = quant_type; all.mode = kFwd;
+    SmallPlan small;
+    if (check_common(all) != TGO_OK) return TGO_E_ARG;
+    if (plan_small(all, small)) return run_small(all, small, static_cast<cudaStream_t>(stream));   // few tokens: all weights in one launch
     // one launch covers two weight sets (their tiles share the launch and the activation rows' L2 residency)
     for (int64_t s = 0; s < num_weights; s += 2) {
         Problem p = {};
