@@ -112,6 +112,18 @@ int tgo_mmq_fwd_multi(const void* x, const void* const* packed_weights, void* co
                       int64_t num_weights, int64_t rows, int64_t out_features, int64_t in_features,
                       int quant_type, void* stream);
 
+/* The chunked LM-head loop: for every chunk of at most chunk_rows rows, logits = hidden * W^T (bf16),
+ * loss += sum over rows of (log-sum-exp - logits[target]) and d_hidden = (softmax - onehot(target)) *
+ * grad_scale * W, with one chunk of logits in the workspace at a time; row sums and the softmax in
+ * fp32, the cotangent rounded to bf16 once.  hidden, d_hidden: [rows, in_features] bf16; targets:
+ * int64 [rows] (a row whose target is outside 0..vocab-1 makes the loss NaN); loss: one float.  The
+ * reference's consumer runs this loop over its dense operators (docs/mmq_bwd_optimization.md:502-524). */
+int64_t tgo_lm_head_loss_workspace_bytes(int64_t rows, int64_t vocab, int64_t in_features, int quant_type,
+                                         int64_t chunk_rows);
+int tgo_lm_head_loss(const void* hidden, const void* packed_weight, const int64_t* targets, int64_t rows,
+                     int64_t vocab, int64_t in_features, int quant_type, int64_t chunk_rows, float grad_scale,
+                     float* loss, void* d_hidden, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* Workspace bytes the grouped calls below need for `rows` routed rows in `num_groups` groups
  * (the device-built tile list; reference: new_grouped_row_task_workspace,
  * csrc/mmq_hip.cu:544-558). */

@@ -11,6 +11,7 @@ import torch  # noqa: F401  (libtorch and the CUDA runtime must be loaded before
 
 try:
     from . import _C  # noqa: F401  registers torch_ggml_ops::* (static registrars run on import)
+    from . import _ext  # noqa: F401  registers their autograd formulas and torch_ggml_ops_b200::*
 except ImportError as exc:  # pragma: no cover - build problem, not a runtime path
     raise ImportError(
         "torch_ggml_ops_b200: the native module is missing or failed to load "

@@ -4,6 +4,7 @@ Produces, next to this file:
 
 * ``lib/libtgo_mmq.so``  - the C-ABI CUDA library (``include/tgo_mmq.h``), compiled by nvcc for
   ``sm_100a`` only (``-gencode arch=compute_100a,code=sm_100a``);
+* ``_ext.abi3.so``       - autograd formulas and this package's own operators (libtorch's C++ API);
 * ``_C.abi3.so``         - the libtorch stable-ABI module that registers the
   ``torch_ggml_ops::*`` operators over that C ABI (reference build recipe: setup.py:23-44,
   ``-DTORCH_TARGET_VERSION=0x020A000000000000 -DTORCH_STABLE_ONLY``).
@@ -32,6 +33,7 @@ BUILD = ROOT / "build"
 LIB_DIR = PKG / "lib"
 LIB_PATH = LIB_DIR / "libtgo_mmq.so"
 SHIM_PATH = PKG / "_C.abi3.so"
+EXT_PATH = PKG / "_ext.abi3.so"
 
 IQ2S_GRID_SHA256 = "e1aa1473412b0552c2174c30ef22ab4073f6a181b85a17056e8249bd2932fd88"
 QUANT_TYPES = (11, 12, 13, 14, 22)
@@ -140,12 +142,33 @@ def build_shim(force: bool = False) -> Path:
     return SHIM_PATH
 
 
+def build_ext(force: bool = False) -> Path:
+    import torch
+
+    src = CSRC / "torch_ext.cpp"
+    if not force and _newer(EXT_PATH, [src, ROOT / "include" / "tgo_mmq.h", LIB_PATH]):
+        return EXT_PATH
+    tdir = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parents[1]
+    inc = [tdir / "include", tdir / "include" / "torch" / "csrc" / "api" / "include", Path(sysconfig.get_paths()["include"]),
+           cuda / "include"]
+    abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
+    _run([_host_cxx(), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}", "-DPy_LIMITED_API=0x030A0000",
+          *[f"-I{p}" for p in inc], str(src), "-o", str(EXT_PATH),
+          f"-L{LIB_DIR}", "-ltgo_mmq", f"-L{tdir / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+          "-Wl,-rpath,$ORIGIN/lib", f"-Wl,-rpath,{tdir / 'lib'}"])
+    return EXT_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> None:
     build_library(force=force, verbose=verbose)
-    build_shim(force=force)
+    with ThreadPoolExecutor(2) as ex:
+        for done in (ex.submit(build_shim, force), ex.submit(build_ext, force)):
+            done.result()
 
 
 if __name__ == "__main__":
     build(force="--force" in sys.argv, verbose="-v" in sys.argv)
     print(LIB_PATH)
     print(SHIM_PATH)
+    print(EXT_PATH)

@@ -540,9 +540,10 @@ static bool plan_small(const Problem& p, SmallPlan& s) {
     // costs a barrier and a pass through shared memory per tile), up to one block per warp where
     // they do not even cover the SMs.
     const int64_t tiles = p.experts == nullptr ? 1 : (p.rows < groups ? p.rows : groups);   // about; the device knows
-    const int64_t row_tiles = tiles * p.nsets * ((p.N + 15) / 16);
+    const int64_t set_tiles = tiles * ((p.N + 15) / 16), row_tiles = set_tiles * p.nsets;
     const int64_t warps = static_cast<int64_t>(num_sms()) * kSmallWarps;
-    int64_t kw = row_tiles > 0 ? (kSmallRounds * warps + row_tiles - 1) / row_tiles : kSmallWarps;
+    // (from one weight set's tiles: a set's results do not depend on the others in the launch)
+    int64_t kw = (kSmallRounds * warps + set_tiles - 1) / set_tiles;
     if (kw > nkb) kw = nkb;
     if (kw > kSmallWarps) kw = kSmallWarps;
     const int64_t rounds = (nkb + kw - 1) / kw;

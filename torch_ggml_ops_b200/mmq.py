@@ -3,7 +3,8 @@
 Same contract as the reference (torch_ggml_ops/mmq.py:4-80): a fake (meta) kernel per operator so
 the ops trace under ``torch.compile``; an autograd formula for ``mmq`` that saves only the packed
 weight and calls ``mmq_grad_input`` on a contiguous cotangent; and a guard that makes second-order
-differentiation of ``mmq_grad_input`` an error.  The packed weight never receives a gradient.
+differentiation of ``mmq_grad_input`` an error (both in ``csrc/torch_ext.cpp``).  The packed weight
+never receives a gradient.
 """
 import torch
 
@@ -22,38 +23,6 @@ def _(input, packed_weight, quant_type, out_features):
 @torch.library.register_fake(f"{_NS}::mmq_grad_input")
 def _(grad_output, packed_weight, quant_type, in_features):
     return _swap_last_dim(grad_output, in_features)
-
-
-def _save_for_dx(ctx, inputs, output) -> None:
-    activation, packed_weight, quant_type, _ = inputs
-    ctx.quant_type = quant_type
-    ctx.in_features = activation.shape[-1]
-    if ctx.needs_input_grad[0]:
-        ctx.save_for_backward(packed_weight)
-
-
-def _dx(ctx, grad_output):
-    if not ctx.needs_input_grad[0]:
-        return None, None, None, None
-    (packed_weight,) = ctx.saved_tensors
-    # The native operator refuses non-contiguous tensors; a cotangent handed over by autograd
-    # may be a transposed view, so only this autograd-owned temporary is normalised.
-    grad_input = torch.ops.torch_ggml_ops.mmq_grad_input.default(
-        grad_output.contiguous(), packed_weight, ctx.quant_type, ctx.in_features)
-    return grad_input, None, None, None
-
-
-torch.library.register_autograd(f"{_NS}::mmq", _dx, setup_context=_save_for_dx)
-
-
-def _no_double_backward(name: str):
-    def backward(ctx, *grads):
-        raise RuntimeError(f"{_NS}::{name} does not support higher-order gradients")
-
-    return backward
-
-
-torch.library.register_autograd(f"{_NS}::mmq_grad_input", _no_double_backward("mmq_grad_input"))
 
 
 def mmq(input: torch.Tensor, packed_weight: torch.Tensor, quant_type: int, out_features: int) -> torch.Tensor:
