@@ -192,6 +192,18 @@ int tgo_route_sort(const int32_t* expert_ids, int64_t n_pairs, int64_t num_exper
                    int32_t* expert_offsets, int32_t* expert_counts, void* workspace,
                    int64_t workspace_bytes, void* stream);
 
+/* One GPU's mixture-of-experts layer, after tgo_route_sort (no counterpart in the reference, whose
+ * rows arrive sorted: csrc/mmq_hip.cu:325-406): pair_row[i] = the pair's row in expert-major buffers of
+ * `capacity` rows (-1: dropped), ends[e] = min(expert_ends[e], capacity), row_weight[row] = pair_weights[i]
+ * (both may be null), *overflow = 1 if some pair had no room, else 0.  tgo_scatter_tokens then writes
+ * token rows src[t] to every row pair_row[t * top_k + s] >= 0; tgo_combine_rows with pair_row adds the
+ * results of a token's pairs. */
+int tgo_local_plan(const int32_t* pair_to_sorted, const int32_t* expert_ends, const float* pair_weights,
+                   int64_t n_pairs, int64_t num_experts, int64_t capacity, int32_t* pair_row, int32_t* ends,
+                   float* row_weight, int32_t* overflow, void* stream);
+int tgo_scatter_tokens(const void* src, const int32_t* pair_row, int64_t tokens, int64_t top_k, void* rows,
+                       int64_t width, void* stream);
+
 /* dst[r][:] = src[index[r] / divisor][:] for bf16 rows of `width` (a multiple of 8); with
  * index = sorted_to_pair and divisor = top_k this builds the expert-sorted activation rows.  An
  * index that is negative, or whose source row is not below src_rows, gives a row of zeros. */

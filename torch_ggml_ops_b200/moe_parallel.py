@@ -124,6 +124,34 @@ class MoEMLPRank:
         self.plan = {"tokens": b["tokens"], "dst_rank": dst_rank, "indices": li, "offsets": lo,
                      "n_rows": lo[self.EL - 1:], "overflow": overflow, "weighted": w is not None}
 
+    # ------------------------------------------------------------------ one rank
+    # With all experts and tokens on one GPU the sorted position of a pair is its row, token rows are
+    # written to their experts' rows straight from the caller's tensor and a token's results are added
+    # straight into the output: no slots, no maps, no token buffers (65536 tokens: 11.96 -> 10.83 ms per step).
+    def local_plan(self, weights: torch.Tensor | None = None) -> None:
+        """``make_plan`` for a world of one rank."""
+        b = self._route
+        w = None if weights is None else weights.reshape(-1).to(torch.float32).contiguous()
+        native.local_plan(b["p2s"], b["eo"], self.cap, b["dst_row"], b["lo"], b["overflow"], pair_weights=w,
+                          row_weight=self.buf["row_weight"])
+        self.plan = {"tokens": b["tokens"], "pair_row": b["dst_row"], "indices": b["ei"], "offsets": b["lo"],
+                     "n_rows": b["lo"][self.E - 1:], "overflow": b["overflow"], "weighted": w is not None}
+
+    def _local_in(self, tokens: torch.Tensor) -> None:
+        if tokens.shape != (self.plan["tokens"], self.H) or tokens.dtype != torch.bfloat16 or not tokens.is_contiguous():
+            raise ValueError(f"expected a contiguous torch.bfloat16 tensor of shape {(self.plan['tokens'], self.H)}")
+        native.scatter_tokens(tokens, self.plan["pair_row"], self.top_k, self.rows_a)
+
+    def local_forward(self, x_tokens: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+        self._local_in(x_tokens)
+        self._experts_forward()
+        return native.combine_rows(self.rows_b, self.plan["pair_row"], self.top_k, out=out)
+
+    def local_grad_input(self, dy_tokens: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+        self._local_in(dy_tokens)
+        self._experts_backward()
+        return native.combine_rows(self.rows_b, self.plan["pair_row"], self.top_k, out=out)
+
     def check_overflow(self) -> None:
         """Raises if the last plan dropped pairs because ``capacity_rows`` was too small (one device
         read: it waits for the stream)."""
@@ -136,15 +164,19 @@ class MoEMLPRank:
 
     def fwd_compute(self) -> None:
         """After every rank's ``fwd_send``: this rank's experts, from token rows to partial sums."""
+        native.ep_expand(self.buf["tok_in"], self.buf["row_slot"], self.plan["n_rows"], self.rows_a)
+        self._experts_forward()
+        native.ep_reduce(self.rows_b, self.buf["slot_rows"], self.top_k, self.buf["y_part"])
+
+    def _experts_forward(self) -> None:
+        """Expert-major rows ``rows_a`` through this rank's experts into ``rows_b``."""
         p = self.plan
         scale = self.buf["row_weight"].reshape(-1) if p["weighted"] else None
-        native.ep_expand(self.buf["tok_in"], self.buf["row_slot"], p["n_rows"], self.rows_a)
         native.grouped_fwd(self.rows_a, self.wg, self.wu, self.gate, self.up, p["indices"], p["offsets"], self.EL,
                            self.cap, self.F, self.H, self.qt_gu, self.ws)
         native.swiglu_fwd(self.gate, self.up, self.h, row_scale=scale, n_rows_device=p["n_rows"])
         native.grouped_fwd(self.h, self.wd, None, self.rows_b, None, p["indices"], p["offsets"], self.EL, self.cap,
                            self.H, self.F, self.qt_d, self.ws)
-        native.ep_reduce(self.rows_b, self.buf["slot_rows"], self.top_k, self.buf["y_part"])
 
     def fwd_recv(self, out: torch.Tensor | None = None) -> torch.Tensor:
         """After every rank's ``fwd_compute``: [tokens, hidden] = sum of the owners' partial sums."""
@@ -157,15 +189,19 @@ class MoEMLPRank:
         native.ep_dispatch_tokens(dy_tokens, self.plan["dst_rank"], self.top_k, self.rank, self.tpr, self.peers["dy_in"])
 
     def bwd_compute(self) -> None:
+        native.ep_expand(self.buf["dy_in"], self.buf["row_slot"], self.plan["n_rows"], self.rows_a)
+        self._experts_backward()
+        native.ep_reduce(self.rows_b, self.buf["slot_rows"], self.top_k, self.buf["dx_part"])
+
+    def _experts_backward(self) -> None:
+        """Cotangent rows ``rows_a`` through this rank's experts into ``rows_b``."""
         p = self.plan
         scale = self.buf["row_weight"].reshape(-1) if p["weighted"] else None
-        native.ep_expand(self.buf["dy_in"], self.buf["row_slot"], p["n_rows"], self.rows_a)
         native.grouped_dx(self.rows_a, None, self.wd, None, self.h, p["indices"], p["offsets"], self.EL, self.cap,
                           self.H, self.F, self.qt_d, self.ws)                       # dh = dy * Wd
         native.swiglu_bwd(self.h, self.gate, self.up, self.dgate, self.dup, row_scale=scale, n_rows_device=p["n_rows"])
         native.grouped_dx(self.dgate, self.dup, self.wg, self.wu, self.rows_b, p["indices"], p["offsets"], self.EL,
                           self.cap, self.F, self.H, self.qt_gu, self.ws)            # dx = dgate * Wg + dup * Wu
-        native.ep_reduce(self.rows_b, self.buf["slot_rows"], self.top_k, self.buf["dx_part"])
 
     def bwd_recv(self, out: torch.Tensor | None = None) -> torch.Tensor:
         dx = out if out is not None else torch.empty(self.plan["tokens"], self.H, dtype=torch.bfloat16, device=self.device)
@@ -234,12 +270,15 @@ class PeerMoEMLP:
             dist.all_gather_into_tensor(self._counts_all, counts, group=self.group)
             counts_all = self._counts_all
         else:
-            counts_all = counts.reshape(1, -1)
+            self.r.local_plan(weights)
+            return
         self.r.make_plan(counts_all, weights)
 
     def forward(self, x_tokens: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """[tokens, hidden] bf16 -> [tokens, hidden]: sum over the token's top-k experts of
         weight * down(silu(gate(x)) * up(x))."""
+        if self.world == 1:
+            return self.r.local_forward(x_tokens, out)
         self.r.fwd_send(x_tokens)
         self._fence()
         self.r.fwd_compute()
@@ -248,6 +287,8 @@ class PeerMoEMLP:
 
     def grad_input(self, dy_tokens: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """Cotangent of ``forward``'s result -> gradient of its input, [tokens, hidden]."""
+        if self.world == 1:
+            return self.r.local_grad_input(dy_tokens, out)
         self.r.bwd_send(dy_tokens)
         self._fence()
         self.r.bwd_compute()

@@ -36,6 +36,8 @@ SIGNATURES = {
     "tgo_grouped_dx": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _i64, _vp]),
     "tgo_route_workspace_bytes": (_i64, [_i64, _i64]),
     "tgo_route_sort": (_i32, [_vp, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp]),
+    "tgo_local_plan": (_i32, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp]),
+    "tgo_scatter_tokens": (_i32, [_vp, _vp, _i64, _i64, _vp, _i64, _vp]),
     "tgo_gather_rows": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _i64, _vp]),
     "tgo_combine_rows": (_i32, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "tgo_quantize_q8": (_i32, [_vp, _i64, _i64, _vp, _vp, _vp, _vp]),
@@ -227,11 +229,24 @@ def gather_rows(src, index, divisor=1, stream=None):
     return dst
 
 
-def combine_rows(rows, pair_to_sorted, top_k, weights=None, stream=None):
+def local_plan(pair_to_sorted, expert_ends, capacity, pair_row, ends, overflow, pair_weights=None, row_weight=None, stream=None) -> None:
+    """Rows, group ends and row weights of one GPU's mixture-of-experts layer (``tgo_local_plan``)."""
+    check(lib().tgo_local_plan(_ptr(pair_to_sorted), _ptr(expert_ends), _ptr(pair_weights), pair_to_sorted.numel(), expert_ends.numel(),
+                               capacity, _ptr(pair_row), _ptr(ends), _ptr(row_weight), _ptr(overflow), _stream(stream)), "tgo_local_plan")
+
+
+def scatter_tokens(src, pair_row, top_k, rows, stream=None) -> None:
+    """rows[pair_row[t * top_k + s]] = src[t] (``tgo_scatter_tokens``)."""
+    check(lib().tgo_scatter_tokens(_ptr(src), _ptr(pair_row), src.shape[0], top_k, _ptr(rows), src.shape[1], _stream(stream)),
+          "tgo_scatter_tokens")
+
+
+def combine_rows(rows, pair_to_sorted, top_k, weights=None, stream=None, out=None):
     import torch
 
     tokens = pair_to_sorted.numel() // top_k
-    out = torch.empty((tokens, rows.shape[1]), dtype=rows.dtype, device=rows.device)
+    if out is None:
+        out = torch.empty((tokens, rows.shape[1]), dtype=rows.dtype, device=rows.device)
     check(lib().tgo_combine_rows(_ptr(rows), _ptr(pair_to_sorted), _ptr(weights), _ptr(out), tokens, top_k,
                                  rows.shape[1], _stream(stream)), "tgo_combine_rows")
     return out
