@@ -350,7 +350,7 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
     constexpr bool k64 = kDecodeWarps == 4;   // a decode thread takes 64 weights (one row of a step)
     // CTA pair: rank 0 (the leader) owns the barriers both CTAs feed (full, acc_empty) and issues
     // the UMMAs; every CTA owns the barriers only it waits on (done, raw, acc_full).
-    const int rank = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;
+    const int rank = CG == 2 ? warp_uniform(static_cast<int>(cluster_ctarank())) : 0;
     const int cta = CG == 2 ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int ncta = CG == 2 ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
@@ -381,7 +381,7 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc_g + kBarBytes);
     volatile int* abort_word = reinterpret_cast<volatile int*>(misc_g + kBarBytes + 4);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_uniform(threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
 
     const int N = args.out_features, K = args.in_features;
@@ -398,7 +398,7 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
     const int steps_all = MODE == kFwd ? steps_set : steps_set * args.nsets;   // steps that hold data
     const int nstages = (nsteps + KS - 1) / KS;                              // decoded stages of a tile
     const int nsteps_pad = nstages * KS;   // a stage's missing steps are fed zeros
-    const int ntasks = args.tasks != nullptr ? *args.task_count : args.dense_tasks;
+    const int ntasks = args.tasks != nullptr ? warp_uniform(*args.task_count) : args.dense_tasks;
     const long long total_tiles = static_cast<long long>(ntasks) * mtiles;
 
     if (threadIdx.x == 0) {
@@ -432,7 +432,7 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
     tc_fence_before_sync();
     if (CG == 2) cluster_sync_all(); else __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = static_cast<uint32_t>(warp_uniform(static_cast<int>(*tmem_slot)));
     // barriers of the leader, as seen from this CTA
     const uint32_t lead_full = CG == 2 ? map_to_cta(bar_full, 0) : bar_full;
     const uint32_t lead_acc_empty = CG == 2 ? map_to_cta(bar_acc_empty, 0) : bar_acc_empty;
@@ -582,14 +582,17 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ UMMA issuer (one thread)
-        // This thread's instruction stream is the serial spine of the kernel: per pipeline stage it
-        // waits once, issues 4 * KS UMMAs and commits once (twice for a pair); every one of these
-        // costs it 50-70 cycles whatever the UMMA's size.  The loop keeps stage counters, barrier
-        // addresses and the low descriptor words as running values (one add per use), and the
-        // narrow kernel's loop body carries nothing of the wide tiles (measured: 4 % of the
-        // forward time).
-        if (lane == 0 && rank == 0) {
+        // ------------------------------------------------------------ UMMA issuer (one warp)
+        // This warp's instruction stream is the serial spine of the kernel: per pipeline stage it waits
+        // once, issues 4 * KS UMMAs and commits once (twice for a pair).  The whole warp walks the loop and
+        // one elected thread issues, so that every operand is warp-uniform and known as such: a UMMA takes
+        // its descriptors from uniform registers, and a loop of one thread (a divergent branch) has to move
+        // each of them there, one by one, every time.  The loop keeps stage counters, barrier addresses and
+        // the low descriptor words as running values (one add per use), and the narrow kernel's loop body
+        // carries nothing of the wide tiles.  ns per tile and 64-element step, Q4_K 512 x 2048, one thread /
+        // whole warp: 32 tokens 390 / 380 forward, 454 / 435 backward; 256 tokens 500 / 495, 627 / 600.
+        if (rank == 0) {
+            const uint32_t elected = elect_one();
             constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);   // SBO 1024, version, SWIZZLE_128B
             constexpr uint32_t kLboA = MODE == kFwd ? 16u : 8192u;                 // forward K-major, backward MN-major
             constexpr uint32_t kStepA = (MODE == kFwd ? 32u : 2048u) >> 4;         // next 16 reduction elements of A
@@ -598,34 +601,34 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
             const uint32_t a_lo0 = ((wgt_s & 0x3FFFFu) >> 4) | ((kLboA >> 4) << 16);
             const uint32_t b_lo0 = ((act_s & 0x3FFFFu) >> 4) | ((16u >> 4) << 16);
             // the peer's copies of the barriers the commits signal
-            const uint32_t peer_done = CG == 2 ? map_to_cta(bar_done, 1) : 0u;
-            const uint32_t peer_acc_full = CG == 2 ? map_to_cta(bar_acc_full, 1) : 0u;
+            const uint32_t peer_done = CG == 2 ? static_cast<uint32_t>(warp_uniform(static_cast<int>(map_to_cta(bar_done, 1)))) : 0u;
+            const uint32_t peer_acc_full = CG == 2 ? static_cast<uint32_t>(warp_uniform(static_cast<int>(map_to_cta(bar_acc_full, 1)))) : 0u;
             uint32_t sa = 0, sb = 0, sbar = 0, ph = 0;   // next decoded-weight slot, activation slot, barrier pair
-            uint32_t full_bar = bar_full, done_bar = bar_done;
             uint32_t tl = 0;   // running accumulator use (a wide tile takes two)
-            bool ok = true, ready = false;
+            bool ok = true;
             for (long long tile = cta; ok && tile < total_tiles; tile += ncta) {
                 TileInfo t;
-                if (!load_tile<MODE, CG, WIDE, SPLIT>(args, static_cast<int>(tile), mtiles, mtiles_set, rank, t)) continue;
+                const bool any = load_tile<MODE, CG, WIDE, SPLIT>(args, static_cast<int>(tile), mtiles, mtiles_set, rank, t);
+                t.ntok = warp_uniform(t.ntok);
+                t.tok0 = warp_uniform(t.tok0);
+                if (!warp_uniform(any)) continue;
                 const uint32_t acc0 = tl & 1u, acc1 = acc0 ^ 1u;
-                if (!mbar_wait(bar_acc_empty + 8 * acc0, ((tl >> 1) & 1u) ^ 1u, abort_word, kAbortAccEmpty)) break;
+                if (!all_wait(bar_acc_empty + 8 * acc0, ((tl >> 1) & 1u) ^ 1u, abort_word, kAbortAccEmpty)) break;
                 tc_fence_after_sync();
                 const uint32_t d_tmem0 = tmem_base + acc0 * kTileTok;
                 const uint32_t idesc0 = umma_idesc_bf16(static_cast<uint32_t>(pad_tokens<CG>(t.tok0)), MODE == kBwd ? 1u : 0u, 0u, 128u * CG);
                 // second half of a wide tile: the other accumulator, its own token count
                 const uint32_t d_tmem1 = tmem_base + acc1 * kTileTok;
                 const uint32_t idesc1 = WIDE ? umma_idesc_bf16(static_cast<uint32_t>(pad_tokens<CG>(t.ntok - t.tok0)), MODE == kBwd ? 1u : 0u, 0u, 128u * CG) : 0u;
-                const int nhalf = WIDE ? t.nhalf : 1;
+                const int nhalf = WIDE && t.ntok > t.tok0 ? 2 : 1;
                 for (int stage = 0; ok && stage < nstages; ++stage) {
                     for (int half = 0; half < nhalf; ++half) {
                         if (WIDE && half == 1 && stage == 0) {   // first use of the second accumulator
-                            if (!mbar_wait(bar_acc_empty + 8 * acc1, (((tl + 1u) >> 1) & 1u) ^ 1u, abort_word, kAbortAccEmpty)) { ok = false; break; }
+                            if (!all_wait(bar_acc_empty + 8 * acc1, (((tl + 1u) >> 1) & 1u) ^ 1u, abort_word, kAbortAccEmpty)) { ok = false; break; }
                             tc_fence_after_sync();
                         }
                         const uint32_t d_tmem = (WIDE && half == 1) ? d_tmem1 : d_tmem0;
                         const uint32_t idesc = (WIDE && half == 1) ? idesc1 : idesc0;
-                        if (!ready && !mbar_wait(full_bar, ph, abort_word, kAbortWgtFull)) { ok = false; break; }
-                        const uint32_t cur_done = done_bar;
                         uint32_t slot_a[KS], slot_b[KS];
                         uint32_t sa_next = sa;
 #pragma unroll
@@ -637,28 +640,24 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
                         }
                         // the decoded steps stay in place until the last half has read them
                         if (half == nhalf - 1) sa = sa_next;
-                        full_bar += 8;
-                        done_bar += 8;
-                        if (++sbar == NB) { sbar = 0; full_bar = bar_full; done_bar = bar_done; ph ^= 1u; }
-                        // with short stages, test the next stage's barrier now: the answer arrives while
-                        // the UMMAs issue; "no" only means "ask again, blocking"
-                        ready = KS == 1 ? mbar_try_wait(full_bar, ph) : false;
+                        if (!all_wait(bar_full + 8 * sbar, ph, abort_word, kAbortWgtFull)) { ok = false; break; }
 #pragma unroll
                         for (uint32_t ks = 0; ks < static_cast<uint32_t>(KS); ++ks) {
                             const uint32_t sa_lo = slot_a[ks], sb_lo = slot_b[ks];
 #pragma unroll
                             for (uint32_t kk = 0; kk < kStepK / 16; ++kk) {
                                 const uint32_t accum = (ks | kk) != 0 ? 1u : (stage != 0 ? 1u : 0u);
-                                if (CG == 2) umma_bf16_lohi_pair(d_tmem, sa_lo + kk * kStepA, sb_lo + kk * kStepB, kDescHi, idesc, accum);
-                                else umma_bf16_lohi(d_tmem, sa_lo + kk * kStepA, sb_lo + kk * kStepB, kDescHi, idesc, accum);
+                                if (CG == 2) umma_bf16_lohi_pair(d_tmem, sa_lo + kk * kStepA, sb_lo + kk * kStepB, kDescHi, idesc, accum, elected);
+                                else umma_bf16_lohi(d_tmem, sa_lo + kk * kStepA, sb_lo + kk * kStepB, kDescHi, idesc, accum, elected);
                             }
                         }
                         if (CG == 2) {
-                            umma_commit_pair(cur_done);
-                            umma_commit_pair(peer_done + (cur_done - bar_done));
+                            umma_commit_pair(bar_done + 8 * sbar, elected);
+                            umma_commit_pair(peer_done + 8 * sbar, elected);
                         } else {
-                            umma_commit(cur_done);
+                            umma_commit(bar_done + 8 * sbar, elected);
                         }
+                        if (++sbar == NB) { sbar = 0; ph ^= 1u; }
                     }
                 }
                 if (ok) {
@@ -666,10 +665,10 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
                     for (int half = 0; half < nhalf; ++half) {
                         const uint32_t acc = half == 0 ? acc0 : acc1;
                         if (CG == 2) {
-                            umma_commit_pair(bar_acc_full + 8 * acc);
-                            umma_commit_pair(peer_acc_full + 8 * acc);
+                            umma_commit_pair(bar_acc_full + 8 * acc, elected);
+                            umma_commit_pair(peer_acc_full + 8 * acc, elected);
                         } else {
-                            umma_commit(bar_acc_full + 8 * acc);
+                            umma_commit(bar_acc_full + 8 * acc, elected);
                         }
                     }
                 }
