@@ -444,7 +444,10 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
     // with two busy warps instead of five; the other partitions take five decode warps each.
     // Measured on the benchmark (Q4_K, 256 ragged groups): forward +3 %; backward, whose short
     // tiles keep the epilogue warps busy, loses with that placement and keeps the plain one.
-    constexpr bool kRemap = MODE == kFwd;
+    // Not for the 2-byte-aligned types: their decode is what sets the pace, and five warps of it on three
+    // partitions cost more than the serial roles gain (ns per tile and step, 512 x 2048, 192 tokens,
+    // with / without: Q6_K 631 / 610, Q3_K 623 / 582, IQ2_S 563 / 536).
+    constexpr bool kRemap = MODE == kFwd && k64;
     constexpr int kActWarp = kRemap ? 5 : 0, kRawWarp = kRemap ? 9 : 2, kRawWarp2 = kRemap ? 13 : 3;
     const bool light = kRemap ? ((warp & 3) == 1 && warp < 16) : warp < kFirstDecodeWarp;
     // decode warp index 0..15
