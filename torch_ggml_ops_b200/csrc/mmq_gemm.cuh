@@ -434,7 +434,7 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
     tc_fence_after_sync();
     const uint32_t tmem_base = static_cast<uint32_t>(warp_uniform(static_cast<int>(*tmem_slot)));
     // barriers of the leader, as seen from this CTA
-    const uint32_t lead_full = CG == 2 ? map_to_cta(bar_full, 0) : bar_full;
+    const uint32_t lead_full = CG == 2 ? static_cast<uint32_t>(warp_uniform(static_cast<int>(map_to_cta(bar_full, 0)))) : bar_full;
     const uint32_t lead_acc_empty = CG == 2 ? map_to_cta(bar_acc_empty, 0) : bar_acc_empty;
 
     // Warp roles.  Backward: warps 0 / 2 / 3 are the activation and the two raw-weight producers,
@@ -457,11 +457,13 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
         // One pipeline stage = KS one-step slots of the tokens of one half.  `it` is the running
         // pipeline-stage index; stage it uses slots it * KS .. it * KS + KS - 1 (mod NBS).
         if (args.use_tma) {
-            if (lane == 0) {
-                for (int s = 0; s < args.nsets; ++s)
-                    for (int b = 0; b < kNumBoxes; ++b) prefetch_tmap(&args.act_maps[s].box[b]);
-                // This thread's loop is one of the serial chains that set the pace, so everything
-                // it needs per stage is a running value: the stage's barrier, the barrier of the
+            {
+                const uint32_t elected = elect_one();
+                if (lane < kNumBoxes) {
+                    for (int s = 0; s < args.nsets; ++s) prefetch_tmap(&args.act_maps[s].box[lane]);
+                }
+                // This loop is one of the serial chains that set the pace (walked by the whole warp, one
+                // elected lane issues: see the UMMA issuer), so everything it needs per stage is a running value: the stage's barrier, the barrier of the
                 // stage whose slots it refills (D stages back), the ring slot, and the position in
                 // the reduction.  The token rows of a half are fetched with the boxes whose heights
                 // are the binary digits of the row count (a multiple of 16).
@@ -477,9 +479,10 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
                     int rem_h[2], row_h[2];
 #pragma unroll
                     for (int h = 0; h < (WIDE ? 2 : 1); ++h) {
-                        rem_h[h] = pad_tokens<CG>(half_tokens(t, h)) / CG;
-                        row_h[h] = half_row0(t, h) + rank * rem_h[h];
+                        rem_h[h] = warp_uniform(pad_tokens<CG>(half_tokens(t, h)) / CG);
+                        row_h[h] = warp_uniform(half_row0(t, h) + rank * rem_h[h]);
                     }
+                    if (WIDE) t.nhalf = warp_uniform(t.nhalf);
                     // position of the tile's next decoded stage in the reduction
                     int step = 0;
                     int astep = SPLIT ? t.split * nsteps : 0;
@@ -494,7 +497,7 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
                         const bool last_half = !(WIDE && t.nhalf == 2) || half == 1;
                         const int rem = rem_h[WIDE ? half : 0], row0 = row_h[WIDE ? half : 0];
                         if (it >= D) {
-                            if (!mbar_wait(bar_done + wait_off, wait_ph, abort_word, kAbortActEmpty)) { ok = false; break; }
+                            if (!all_wait(bar_done + wait_off, wait_ph, abort_word, kAbortActEmpty)) { ok = false; break; }
                             wait_off += 8;
                             if (wait_off == 8 * NB) { wait_off = 0; wait_ph ^= 1u; }
                         }
@@ -502,7 +505,7 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
                         // of the token rows (all of them, or its half) and the bytes count on the
                         // leader's barrier
                         const uint32_t bar = lead_full + full_off;
-                        if (rank == 0) mbar_arrive_expect_tx(bar_full + full_off, static_cast<uint32_t>(rem * CG) * 128u * KS);
+                        if (rank == 0) mbar_arrive_expect_tx(bar_full + full_off, static_cast<uint32_t>(rem * CG) * 128u * KS, elected);
                         int s_step = step, s_astep = astep, s_set = set, s_red = red0;
 #pragma unroll
                         for (int ks = 0; ks < KS; ++ks) {
@@ -517,8 +520,8 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
                                 const int h = 256 >> b;
                                 if (h <= Cfg::kActRows && (rem & h) != 0) {
                                     const int off = rem & (kAll & ~(2 * h - 1));   // rows taken by the taller boxes
-                                    if (CG == 2) tma_load_2d_pair(dst + off * 128, &args.act_maps[use_set].box[b], bar, col, row0 + off);
-                                    else tma_load_2d(dst + off * 128, &args.act_maps[use_set].box[b], bar, col, row0 + off);
+                                    if (CG == 2) tma_load_2d_pair(dst + off * 128, &args.act_maps[use_set].box[b], bar, col, row0 + off, elected);
+                                    else tma_load_2d(dst + off * 128, &args.act_maps[use_set].box[b], bar, col, row0 + off, elected);
                                 }
                             }
                             if (++slot == NBS) slot = 0;
@@ -685,7 +688,8 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
         // some 900 cycles per stage (a wait, an expect_tx, the copies, each a shared-memory or TMA
         // round trip under load), which backward - one raw stage per 64-element step - set the pace.
         const uint32_t my_parity = warp == kRawWarp ? 0u : 1u;
-        if (lane == 0) {
+        {
+            const uint32_t elected = elect_one();
             uint32_t itr = 0;
             bool ok = true;
             const int P = args.wgt_classes, lgP = args.wgt_classes_log2;
@@ -704,7 +708,7 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
                 TileInfo t;
                 if (!load_tile<MODE, CG, WIDE, SPLIT>(args, static_cast<int>(tile), mtiles, mtiles_set, rank, t)) continue;
                 const int nraw = MODE == kFwd ? nkb : nsteps_pad;
-                const long long gbase = static_cast<long long>(t.expert) * N + (MODE == kFwd ? t.m0 : 0);
+                const long long gbase = static_cast<long long>(warp_uniform(t.expert)) * N + (MODE == kFwd ? t.m0 : 0);
                 int y0[kMaxWgtClasses], x0[kMaxWgtClasses];
 #pragma unroll
                 for (int c = 0; c < kMaxWgtClasses; ++c) {
@@ -733,7 +737,7 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
                         continue;
                     }
                     const uint32_t r = itr % NR, ph = (itr / NR) & 1u;
-                    if (!mbar_wait(bar_raw_empty + 8 * r, ph ^ 1u, abort_word, kAbortRawEmpty)) { ok = false; break; }
+                    if (!all_wait(bar_raw_empty + 8 * r, ph ^ 1u, abort_word, kAbortRawEmpty)) { ok = false; break; }
                     int use_set = set, yoff = 0, xoff = 0;
                     if (MODE == kFwd) {
                         xoff = ri * Fmt::kBytes;
@@ -742,13 +746,13 @@ mmq_gemm_kernel(const __grid_constant__ GemmArgs args) {
                         if (ri >= nsteps || astep >= steps_all) { use_set = 0; yoff = 0; }   // a step past the end: decoded as zeros
                     }
                     const uint32_t bar = bar_raw_full + 8 * r;
-                    mbar_arrive_expect_tx(bar, tx_bytes);
+                    mbar_arrive_expect_tx(bar, tx_bytes, elected);
                     const uint32_t stage_s = raw_s + r * Cfg::kRawStageBytes;
 #pragma unroll
                     for (int c = 0; c < kMaxWgtClasses; ++c) {
                         if (c < P)
                             tma_load_2d(stage_s + c * rows_per_class * Fmt::kBox, &args.wgt_maps[use_set].cls[c], bar,
-                                        (x0[c] + xoff) & ~15, y0[c] + yoff);
+                                        (x0[c] + xoff) & ~15, y0[c] + yoff, elected);
                     }
                     if (MODE == kBwd) {
                         ++astep;
