@@ -137,3 +137,28 @@ def test_short_reductions_and_wide_tiles(cuda, monkeypatch):
         assert np.array_equal(bits(narrow), bits(wide)), N
         assert ref.rel_frobenius(wide.float().cpu(), ref.grouped_grad_input(dy, W, ids, eo)) < DX_TOL
     assert native.device_status() == 0
+
+
+@pytest.mark.parametrize("name,qt", ALL_TYPES)
+@pytest.mark.parametrize("mean,K", [(255, 1024), (256, 1024), (256, 768), (1023, 768), (1024, 768)])
+def test_grouped_choice_of_tile_width(cuda, monkeypatch, name, qt, mean, K):
+    """Either side of the rows per group and reduction length at which wide tiles are chosen: the
+    calls as made (no override) give the bits of 256-token tiles, whatever their width."""
+    import torch_ggml_ops_b200 as tgo
+
+    E, N = 3, 256
+    sizes = [mean - 200, mean + 201, mean - 1]   # their mean is `mean`, none of them is
+    w, _ = expert_case(qt, E, N, K, 6)
+    ei, eo = routing_from_sizes(sizes, [2, 0, 1])
+    xd, dyd, wd = to_dev(blocks.gaussian_bf16((3 * mean, K), 7)), to_dev(blocks.gaussian_bf16((3 * mean, N), 8)), to_dev(w)
+    eid, eod = to_dev(ei), to_dev(eo)
+
+    def run():
+        x = xd.detach().requires_grad_(True)
+        y = tgo.grouped_mmq(x, wd, eid, eod, qt, N)
+        return y, torch.autograd.grad(y, x, dyd)[0]
+
+    auto = run()
+    monkeypatch.setenv("TGO_WIDE_TILES", "0")
+    narrow = run()
+    assert all(np.array_equal(bits(a.detach()), bits(n.detach())) for a, n in zip(auto, narrow))

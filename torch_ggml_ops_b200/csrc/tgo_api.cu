@@ -459,6 +459,24 @@ struct Problem {
     void* const* out_rows;    // forward, one weight set: per-row destinations instead of out[0]
 };
 
+// Tiles of up to 512 tokens (two accumulators sharing each decoded weight step) halve the decode work
+// per output element and the number of tiles.  Dense: whenever the 256-token tiles would not all run at
+// once (and there are more than 256 tokens to share a step).  Grouped: ragged groups leave wide tiles
+// part empty and the coarser tiles balance worse, so it takes a costly decode and enough rows per group
+// (us, narrow / wide, B200, 256 experts, skewed groups):
+//                         mean rows          128       256        512        1024       2048
+//   Q6_K 512 x 2048 forward                210/169    245/222    394/319    632/519   1249/924
+//   IQ2_S gate/up pair, input gradient     331/335    465/398    707/566   1290/1039  2544/2228
+//   IQ2_S 2048 x 512 forward               169/181    247/235    394/392    703/642   1243/1175
+//   Q3_K 2048 x 512 forward                177/194    253/265    381/382    687/648   1306/1248
+// A forward tile of few steps spends its time in the epilogue, which wide tiles do not shorten.
+// TGO_WIDE_TILES overrides the choice (tests run every case both ways); results are the same bits.
+static bool wide_groups(const Problem& p) {
+    if (p.qt == QT_Q4_K || p.qt == QT_Q5_K) return false;   // the cheap decode of the 16-byte-aligned types
+    const int64_t least = p.mode == kFwd && p.K < 16 * kStepK ? 1024 : 256;
+    return p.rows >= least * p.groups;
+}
+
 static int check_common(const Problem& p) {
     const int64_t bb = tgo_block_bytes(p.qt);
     if (bb < 0) return fail(TGO_E_ARG, "unsupported quant_type: %d", p.qt);
@@ -650,14 +668,9 @@ static int run_problem(const Problem& p, cudaStream_t stream) {
     const int64_t tile_m = static_cast<int64_t>(kTileM) * cg;
     const int64_t mtiles = p.mode == kFwd ? ((p.N + tile_m - 1) / tile_m) * p.nsets : p.K / tile_m;
     const int64_t limit = cg == 2 ? pairs : num_sms();
-    // Tiles of up to 512 tokens (two accumulators sharing each decoded weight step) halve the
-    // decode work per output element and the number of tiles.  Measured on B200 (Q4_K): dense
-    // M = 4096 gains 11 % forward and 20 % backward once the 256-token tiles no longer all run at
-    // once; grouped inputs lose 3-10 % whatever the mean group size (256, 512 or 2048 rows), because
-    // ragged groups leave the wide tiles part empty and the coarser tiles balance worse.  So: dense
-    // inputs only.  TGO_WIDE_TILES overrides the choice (tests run every case both ways).
     const int wide_env = wide_tiles_env();
-    bool wide = p.experts == nullptr && ((p.rows + kTileTok - 1) / kTileTok) * mtiles > limit;
+    bool wide = p.experts == nullptr ? p.rows > kTileTok && ((p.rows + kTileTok - 1) / kTileTok) * mtiles > limit
+                                     : wide_groups(p);
     if (wide_env >= 0) wide = wide_env != 0;
     int max_tok = wide ? kWideTok : kTileTok;
     // split reduction: dense input gradient of a single weight with a workspace to hold the partial sums
