@@ -140,7 +140,7 @@ def test_short_reductions_and_wide_tiles(cuda, monkeypatch):
 
 
 @pytest.mark.parametrize("name,qt", ALL_TYPES)
-@pytest.mark.parametrize("mean,K", [(255, 1024), (256, 1024), (256, 768), (1023, 768), (1024, 768)])
+@pytest.mark.parametrize("mean,K", [(255, 1024), (256, 1024), (256, 768), (511, 768), (512, 768), (512, 1024)])
 def test_grouped_choice_of_tile_width(cuda, monkeypatch, name, qt, mean, K):
     """Either side of the rows per group and reduction length at which wide tiles are chosen: the
     calls as made (no override) give the bits of 256-token tiles, whatever their width."""

@@ -462,18 +462,23 @@ struct Problem {
 // Tiles of up to 512 tokens (two accumulators sharing each decoded weight step) halve the decode work
 // per output element and the number of tiles.  Dense: whenever the 256-token tiles would not all run at
 // once (and there are more than 256 tokens to share a step).  Grouped: ragged groups leave wide tiles
-// part empty and the coarser tiles balance worse, so it takes a costly decode and enough rows per group
+// part empty and the coarser tiles balance worse, so it takes enough rows per group, more for the cheap
+// decode of the 16-byte-aligned types, which gain in no size backward
 // (us, narrow / wide, B200, 256 experts, skewed groups):
 //                         mean rows          128       256        512        1024       2048
 //   Q6_K 512 x 2048 forward                210/169    245/222    394/319    632/519   1249/924
 //   IQ2_S gate/up pair, input gradient     331/335    465/398    707/566   1290/1039  2544/2228
 //   IQ2_S 2048 x 512 forward               169/181    247/235    394/392    703/642   1243/1175
 //   Q3_K 2048 x 512 forward                177/194    253/265    381/382    687/648   1306/1248
+//   Q5_K gate/up pair, forward                        396/394    633/587   1035/890   2009/2021
+//   Q4_K 2048 x 512 forward                           228/249    392/353    646/632   1393/1340
+//   Q4_K 512 x 2048 input gradient                    173/206    303/321    564/580   1115/1336
 // A forward tile of few steps spends its time in the epilogue, which wide tiles do not shorten.
 // TGO_WIDE_TILES overrides the choice (tests run every case both ways); results are the same bits.
 static bool wide_groups(const Problem& p) {
-    if (p.qt == QT_Q4_K || p.qt == QT_Q5_K) return false;   // the cheap decode of the 16-byte-aligned types
-    const int64_t least = p.mode == kFwd && p.K < 16 * kStepK ? 1024 : 256;
+    const bool cheap = p.qt == QT_Q4_K || p.qt == QT_Q5_K;
+    if (p.mode == kBwd && cheap) return false;
+    const int64_t least = cheap || (p.mode == kFwd && p.K < 16 * kStepK) ? 512 : 256;
     return p.rows >= least * p.groups;
 }
 
