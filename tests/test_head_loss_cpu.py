@@ -1,0 +1,53 @@
+"""The autograd side of ``lm_head_loss`` (csrc/torch_ext.cpp) without a GPU: the operator's CUDA kernel is
+stood in for by a plain CPU one, everything above it is the package's own."""
+import pytest
+import torch
+
+V, K, T = 40, 16, 12
+
+
+def _weight(w):
+    return w.view(-1).float()[: V * K].reshape(V, K) / 128 - 1
+
+
+def _loss(h, w, quant_type, vocab, targets, chunk_rows, grad_scale):
+    lp = torch.log_softmax(h.float() @ _weight(w).t(), -1)
+    loss = -lp.gather(1, targets[:, None]).sum()
+    d = lp.exp().scatter_add_(1, targets[:, None], torch.full((h.shape[0], 1), -1.0)) * grad_scale
+    return loss, (d @ _weight(w)).to(h.dtype)
+
+
+@pytest.fixture
+def head():
+    import torch_ggml_ops_b200 as tgo
+
+    lib = torch.library.Library("torch_ggml_ops_b200", "IMPL")
+    lib.impl("lm_head_loss", _loss, "CPU")
+    g = torch.Generator().manual_seed(1)
+    w = torch.randint(0, 256, (V * K,), dtype=torch.uint8, generator=g)
+    hidden = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    targets = torch.randint(0, V, (T,), generator=g)
+    yield hidden, lambda h, **kw: tgo.lm_head_loss(h, w, 14, V, targets, **kw)
+    lib._destroy()
+
+
+def test_second_derivatives_are_refused(head):
+    """The loss is not linear in hidden: a gradient without a graph would silently lose its Hessian."""
+    hidden, loss_of = head
+    x = hidden.clone().requires_grad_()
+    (dx,) = torch.autograd.grad(loss_of(x)[0], x, create_graph=True)
+    assert dx.requires_grad
+    with pytest.raises(RuntimeError, match="higher-order"):
+        torch.autograd.grad((x ** 2).sum().float() + (dx.float() ** 2).sum(), x)
+    # neither with respect to the cotangent
+    y = hidden.clone().requires_grad_()
+    with pytest.raises(RuntimeError, match="higher-order"):
+        (dy,) = torch.autograd.grad(loss_of(y)[0] ** 2, y, create_graph=True)
+        dy.float().sum().backward()
+    # a first derivative is not affected, and hidden may change once the loss has been computed
+    z = hidden.clone().requires_grad_()
+    h = z * 1
+    loss = loss_of(h)[0]
+    h.add_(1)
+    loss.backward()
+    assert torch.equal(z.grad, dx.detach())

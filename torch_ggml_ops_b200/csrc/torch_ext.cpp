@@ -379,14 +379,26 @@ std::tuple<Tensor, Tensor> call_lm_head(const Tensor& x, const Tensor& w, int64_
         "torch_ggml_ops_b200::lm_head_loss");
     return h.call(x, w, qt, vocab, t, chunk, scale);
 }
-// The gradient of the loss is the one the call has computed, without its scale.
+// d * g * scale, the gradient that autograd gets.  The loss is not linear in hidden and d has no graph, so
+// a second derivative is refused; `edge` ties the result to hidden for that.
+struct LmHeadGradFn : public Function<LmHeadGradFn> {
+    static Tensor forward(AutogradContext*, const Tensor& edge, const Tensor& d, const Tensor& g, double scale) {
+        at::AutoDispatchBelowADInplaceOrView guard;
+        return (d.to(at::kFloat) * (g * scale)).to(d.scalar_type());
+    }
+    static tensor_list backward(AutogradContext*, tensor_list) {
+        TORCH_CHECK(false, "torch_ggml_ops_b200::lm_head_loss does not support higher-order gradients");
+    }
+};
+// The gradient of the loss is the one the call has computed, without its scale.  `edge`: an empty tensor
+// whose history is hidden's (hidden itself is not kept, so it may be overwritten before the backward pass).
 struct LmHeadFn : public Function<LmHeadFn> {
-    static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, int64_t qt, int64_t vocab, const Tensor& t, int64_t chunk,
-                                 double scale) {
+    static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& edge, const Tensor& w, int64_t qt, int64_t vocab,
+                                 const Tensor& t, int64_t chunk, double scale) {
         at::AutoDispatchBelowADInplaceOrView guard;
         auto [loss, d] = call_lm_head(x, w, qt, vocab, t, chunk, scale);
         Tensor unscaled = scale != 0.0 ? d : std::get<1>(call_lm_head(x, w, qt, vocab, t, chunk, 1.0));
-        ctx->save_for_backward({unscaled});
+        ctx->save_for_backward({unscaled, edge});
         ctx->saved_data["scale"] = scale != 0.0 ? 1.0 / scale : 1.0;
         ctx->mark_non_differentiable({d});
         return {loss, d};
@@ -394,15 +406,16 @@ struct LmHeadFn : public Function<LmHeadFn> {
     static tensor_list backward(AutogradContext* ctx, tensor_list g) {
         Tensor dx;
         if (ctx->needs_input_grad(0) && g[0].defined()) {
-            const Tensor d = ctx->get_saved_variables()[0];
-            dx = (d.to(at::kFloat) * (g[0] * ctx->saved_data["scale"].toDouble())).to(d.scalar_type());
+            const variable_list s = ctx->get_saved_variables();
+            dx = LmHeadGradFn::apply(s[1], s[0], g[0], ctx->saved_data["scale"].toDouble());
         }
-        return {dx, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+        return {dx, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 std::tuple<Tensor, Tensor> lm_head_autograd(const Tensor& x, const Tensor& w, int64_t qt, int64_t vocab, const Tensor& t, int64_t chunk, double scale) {
     if (wants_grad(x)) {
-        const variable_list r = LmHeadFn::apply(x, w, qt, vocab, t, chunk, scale);
+        TORCH_CHECK(x.dim() == 2, "hidden must have shape [rows, in_features]");
+        const variable_list r = LmHeadFn::apply(x, x.narrow(0, 0, 0).clone(), w, qt, vocab, t, chunk, scale);
         return {r[0], r[1]};
     }
     at::AutoDispatchBelowADInplaceOrView guard;
