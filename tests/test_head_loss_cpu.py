@@ -51,3 +51,12 @@ def test_second_derivatives_are_refused(head):
     h.add_(1)
     loss.backward()
     assert torch.equal(z.grad, dx.detach())
+
+
+def test_a_derivative_of_the_returned_gradient_is_refused(head):
+    hidden, loss_of = head
+    x = hidden.clone().requires_grad_()
+    loss, d = loss_of(x)
+    assert d.requires_grad
+    with pytest.raises(RuntimeError, match="higher-order"):
+        torch.autograd.grad(loss + d.float().sum(), x)

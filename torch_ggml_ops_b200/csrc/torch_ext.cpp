@@ -379,6 +379,7 @@ std::tuple<Tensor, Tensor> call_lm_head(const Tensor& x, const Tensor& w, int64_
         "torch_ggml_ops_b200::lm_head_loss");
     return h.call(x, w, qt, vocab, t, chunk, scale);
 }
+[[noreturn]] void no_second_order_head() { TORCH_CHECK(false, "torch_ggml_ops_b200::lm_head_loss does not support higher-order gradients"); }
 // d * g * scale, the gradient that autograd gets.  The loss is not linear in hidden and d has no graph, so
 // a second derivative is refused; `edge` ties the result to hidden for that.
 struct LmHeadGradFn : public Function<LmHeadGradFn> {
@@ -386,9 +387,7 @@ struct LmHeadGradFn : public Function<LmHeadGradFn> {
         at::AutoDispatchBelowADInplaceOrView guard;
         return (d.to(at::kFloat) * (g * scale)).to(d.scalar_type());
     }
-    static tensor_list backward(AutogradContext*, tensor_list) {
-        TORCH_CHECK(false, "torch_ggml_ops_b200::lm_head_loss does not support higher-order gradients");
-    }
+    static tensor_list backward(AutogradContext*, tensor_list) { no_second_order_head(); }
 };
 // The gradient of the loss is the one the call has computed, without its scale.  `edge`: an empty tensor
 // whose history is hidden's (hidden itself is not kept, so it may be overwritten before the backward pass).
@@ -400,11 +399,12 @@ struct LmHeadFn : public Function<LmHeadFn> {
         Tensor unscaled = scale != 0.0 ? d : std::get<1>(call_lm_head(x, w, qt, vocab, t, chunk, 1.0));
         ctx->save_for_backward({unscaled, edge});
         ctx->saved_data["scale"] = scale != 0.0 ? 1.0 / scale : 1.0;
-        ctx->mark_non_differentiable({d});
+        ctx->set_materialize_grads(false);
         return {loss, d};
     }
     static tensor_list backward(AutogradContext* ctx, tensor_list g) {
         Tensor dx;
+        if (g[1].defined()) no_second_order_head();   // d is a derivative already
         if (ctx->needs_input_grad(0) && g[0].defined()) {
             const variable_list s = ctx->get_saved_variables();
             dx = LmHeadGradFn::apply(s[1], s[0], g[0], ctx->saved_data["scale"].toDouble());
