@@ -123,6 +123,12 @@ int64_t tgo_lm_head_loss_workspace_bytes(int64_t rows, int64_t vocab, int64_t in
 int tgo_lm_head_loss(const void* hidden, const void* packed_weight, const int64_t* targets, int64_t rows,
                      int64_t vocab, int64_t in_features, int quant_type, int64_t chunk_rows, float grad_scale,
                      float* loss, void* d_hidden, void* workspace, int64_t workspace_bytes, void* stream);
+/* The same call, which also writes d_hidden before its rounding to bf16 (fp32, 16-byte aligned, may be null):
+ * what a caller multiplies by the cotangent of the loss, so that the product is rounded once. */
+int tgo_lm_head_loss_f32(const void* hidden, const void* packed_weight, const int64_t* targets, int64_t rows,
+                         int64_t vocab, int64_t in_features, int quant_type, int64_t chunk_rows, float grad_scale,
+                         float* loss, void* d_hidden, float* d_hidden_f32, void* workspace, int64_t workspace_bytes,
+                         void* stream);
 
 /* Workspace bytes the grouped calls below need for `rows` routed rows in `num_groups` groups
  * (the device-built tile list; reference: new_grouped_row_task_workspace,

@@ -14,7 +14,8 @@ def _loss(h, w, quant_type, vocab, targets, chunk_rows, grad_scale):
     lp = torch.log_softmax(h.float() @ _weight(w).t(), -1)
     loss = -lp.gather(1, targets[:, None]).sum()
     d = lp.exp().scatter_add_(1, targets[:, None], torch.full((h.shape[0], 1), -1.0)) * grad_scale
-    return loss, (d @ _weight(w)).to(h.dtype)
+    d = d @ _weight(w)
+    return loss, d.to(h.dtype), d
 
 
 @pytest.fixture
@@ -22,7 +23,8 @@ def head():
     import torch_ggml_ops_b200 as tgo
 
     lib = torch.library.Library("torch_ggml_ops_b200", "IMPL")
-    lib.impl("lm_head_loss", _loss, "CPU")
+    lib.impl("lm_head_loss", lambda *a: _loss(*a)[:2], "CPU")
+    lib.impl("lm_head_loss_f32", _loss, "CPU")
     g = torch.Generator().manual_seed(1)
     w = torch.randint(0, 256, (V * K,), dtype=torch.uint8, generator=g)
     hidden = torch.randn(T, K, generator=g).to(torch.bfloat16)
@@ -60,3 +62,24 @@ def test_a_derivative_of_the_returned_gradient_is_refused(head):
     assert d.requires_grad
     with pytest.raises(RuntimeError, match="higher-order"):
         torch.autograd.grad(loss + d.float().sum(), x)
+
+
+@pytest.mark.parametrize("grad_scale", [1.0, 0.3, 3.0, 0.0, 1e-45, 1e38])
+def test_the_gradient_is_rounded_once(head, grad_scale):
+    """cotangent * gradient in fp32, then one rounding: at most half a unit in the last of bf16's 8 significant
+    bits, 2^-9 of a value's power of two (a thousandth of it is left to the fp32 products)."""
+    hidden, loss_of = head
+    for cotangent in (1.0, 0.37, -1.0 / 3.0, 1e-3):
+        x = hidden.clone().requires_grad_()
+        loss, d = loss_of(x, grad_scale=grad_scale)
+        with torch.no_grad():
+            d.mul_(2)   # the caller's copy is the caller's
+        (loss * cotangent).backward()
+        y = hidden.double().requires_grad_()
+        w = _weight(torch.randint(0, 256, (V * K,), dtype=torch.uint8, generator=torch.Generator().manual_seed(1)))
+        g = torch.Generator().manual_seed(1)
+        torch.randint(0, 256, (V * K,), dtype=torch.uint8, generator=g), torch.randn(T, K, generator=g)
+        targets = torch.randint(0, V, (T,), generator=g)
+        (torch.nn.functional.cross_entropy(y @ w.double().t(), targets, reduction="sum") * cotangent).backward()
+        unit = torch.exp2(torch.floor(torch.log2(y.grad.abs())) - 7)
+        assert bool(((x.grad.double() - y.grad).abs() <= 0.501 * unit + 1e-6 * y.grad.abs().max()).all())

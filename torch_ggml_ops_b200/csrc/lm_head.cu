@@ -16,6 +16,8 @@
 namespace tgo {
 
 int route_fail(int code, const char* msg);  // tgo_api.cu
+int mmq_dx_f32(const void* dy, const void* packed_weight, void* dx, float* dx_f32, int64_t rows, int64_t out_features, int64_t in_features,
+               int quant_type, void* workspace, int64_t workspace_bytes, void* stream);  // tgo_api.cu
 
 constexpr int kXentThreads = 256;
 constexpr int kXentMaxSplits = 16;   // parts of a row in the statistics pass
@@ -194,9 +196,9 @@ int64_t tgo_lm_head_loss_workspace_bytes(int64_t rows, int64_t vocab, int64_t in
     return head_space(rows, vocab, in_features, quant_type, chunk_rows < rows ? chunk_rows : rows).total;
 }
 
-int tgo_lm_head_loss(const void* hidden, const void* packed_weight, const int64_t* targets, int64_t rows, int64_t vocab,
-                     int64_t in_features, int quant_type, int64_t chunk_rows, float grad_scale, float* loss, void* d_hidden,
-                     void* workspace, int64_t workspace_bytes, void* stream) {
+int tgo_lm_head_loss_f32(const void* hidden, const void* packed_weight, const int64_t* targets, int64_t rows, int64_t vocab,
+                         int64_t in_features, int quant_type, int64_t chunk_rows, float grad_scale, float* loss, void* d_hidden,
+                         float* d_hidden_f32, void* workspace, int64_t workspace_bytes, void* stream) {
     if (targets == nullptr || loss == nullptr || workspace == nullptr) return route_fail(TGO_E_ARG, "null pointer");
     if (chunk_rows <= 0) return route_fail(TGO_E_ARG, "chunk_rows must be positive");
     if (rows <= 0) return route_fail(TGO_E_ARG, "zero-row inputs are not supported");
@@ -226,12 +228,20 @@ int tgo_lm_head_loss(const void* hidden, const void* packed_weight, const int64_
                                                             grad_scale, row_loss + b + r);
         }
         if (cudaGetLastError() != cudaSuccess) return route_fail(TGO_E_CUDA, "cross-entropy kernel launch failed");
-        rc = tgo_mmq_dx_ws(logits, packed_weight, static_cast<__nv_bfloat16*>(d_hidden) + b * in_features, n, vocab, in_features, quant_type,
-                           ws + sp.dx_ws, sp.total - sp.dx_ws, stream);
+        rc = mmq_dx_f32(logits, packed_weight, static_cast<__nv_bfloat16*>(d_hidden) + b * in_features,
+                        d_hidden_f32 != nullptr ? d_hidden_f32 + b * in_features : nullptr, n, vocab, in_features, quant_type, ws + sp.dx_ws,
+                        sp.total - sp.dx_ws, stream);
         if (rc != TGO_OK) return rc;
     }
     sum_rows_kernel<<<1, 256, 0, st>>>(row_loss, rows, loss);
     return cudaGetLastError() == cudaSuccess ? TGO_OK : route_fail(TGO_E_CUDA, "sum_rows_kernel launch failed");
+}
+
+int tgo_lm_head_loss(const void* hidden, const void* packed_weight, const int64_t* targets, int64_t rows, int64_t vocab,
+                     int64_t in_features, int quant_type, int64_t chunk_rows, float grad_scale, float* loss, void* d_hidden,
+                     void* workspace, int64_t workspace_bytes, void* stream) {
+    return tgo_lm_head_loss_f32(hidden, packed_weight, targets, rows, vocab, in_features, quant_type, chunk_rows, grad_scale, loss, d_hidden,
+                                nullptr, workspace, workspace_bytes, stream);
 }
 
 }  // extern "C"

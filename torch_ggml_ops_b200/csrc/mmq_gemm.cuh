@@ -145,7 +145,7 @@ struct GemmArgs {
     // are cut into nsplit ranges of split_steps 64-element steps, each tile reduces one range and
     // writes fp32 partial sums [split][row][k] to `partial`; a second kernel adds them in order.
     float* partial;                      // null: no split
-    int nsplit;                          // 1: no split
+    int nsplit;                          // 1: no split (with `partial`: one range, its sums are the fp32 result)
     int split_steps;                     // steps per split (a multiple of the steps per stage)
     // Forward of one weight set with scattered output rows: out_rows[r] is where row r of the result
     // goes (any address this GPU can store to - its own memory or a peer's - 16-byte aligned, or null

@@ -60,7 +60,7 @@ static int launch_one(const GemmArgs& args, int grid, cudaStream_t stream) {
 // the kernel variant for this launch: wide tiles, or (backward only) a split reduction, or neither
 template <int QT, int MODE, int CG>
 static int launch_width(int wide, const GemmArgs& args, int grid, cudaStream_t stream) {
-    if (MODE == kBwd && args.nsplit > 1) return launch_one<QT, kBwd, CG, 0, 1>(args, grid, stream);
+    if (MODE == kBwd && args.partial != nullptr) return launch_one<QT, kBwd, CG, 0, 1>(args, grid, stream);
     return wide ? launch_one<QT, MODE, CG, 1, 0>(args, grid, stream) : launch_one<QT, MODE, CG, 0, 0>(args, grid, stream);
 }
 

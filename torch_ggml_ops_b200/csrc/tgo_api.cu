@@ -347,15 +347,17 @@ __global__ void __launch_bounds__(64) wait_selftest_kernel(long long limit_cycle
 }
 
 // ------------------------------------------------------------------ split-reduction epilogue
-// out[i] = bf16(sum over splits s, in ascending order, of partial[s][i]); four elements per thread.
+// out[i] = bf16(sum over splits s, in ascending order, of partial[s][i]); four elements per thread.  out_f32,
+// if given, receives the sum itself.
 __global__ void __launch_bounds__(256) split_reduce_kernel(const float4* __restrict__ partial, int nsplit, long long n_vec,
-                                                           uint2* __restrict__ out) {
+                                                           uint2* __restrict__ out, float4* __restrict__ out_f32) {
     for (long long v = blockIdx.x * 256LL + threadIdx.x; v < n_vec; v += 256LL * gridDim.x) {
         float4 acc = partial[v];
         for (int s = 1; s < nsplit; ++s) {
             const float4 p = partial[s * n_vec + v];
             acc.x += p.x; acc.y += p.y; acc.z += p.z; acc.w += p.w;
         }
+        if (out_f32 != nullptr) out_f32[v] = acc;
         const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
         out[v] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
     }
@@ -457,6 +459,7 @@ struct Problem {
     void* ws;
     int64_t ws_bytes;
     void* const* out_rows;    // forward, one weight set: per-row destinations instead of out[0]
+    float* out_f32;           // dense input gradient of one weight with a workspace: the result before its rounding as well
 };
 
 // Tiles of up to 512 tokens (two accumulators sharing each decoded weight step) halve the decode work
@@ -680,19 +683,21 @@ static int run_problem(const Problem& p, cudaStream_t stream) {
     int max_tok = wide ? kWideTok : kTileTok;
     // split reduction: dense input gradient of a single weight with a workspace to hold the partial sums
     int nsplit = 1, split_steps = 0;
-    if (p.experts == nullptr && p.mode == kBwd && p.nsets == 1 && p.ws != nullptr && wide_env < 0) {
-        nsplit = plan_split(p.rows, p.N, p.K, tile_m, limit, split_steps);
+    if (p.experts == nullptr && p.mode == kBwd && p.nsets == 1 && p.ws != nullptr) {
+        if (wide_env < 0) nsplit = plan_split(p.rows, p.N, p.K, tile_m, limit, split_steps);
         if (nsplit > 1) {
             const int64_t need = static_cast<int64_t>(nsplit) * p.rows * p.K * 4;
             if (p.ws_bytes < need) return fail(TGO_E_WORKSPACE, "workspace has %lld bytes, need %lld", (long long)p.ws_bytes, (long long)need);
             if (!aligned16(p.ws)) return fail(TGO_E_ARG, "workspace pointer must be 16-byte aligned");
+        }
+        if (nsplit > 1 || p.out_f32 != nullptr) {
             wide = false;
             max_tok = kTileTok;
         }
     }
     a.nsplit = nsplit;
     a.split_steps = split_steps;
-    a.partial = nsplit > 1 ? static_cast<float*>(p.ws) : nullptr;
+    a.partial = nsplit > 1 ? static_cast<float*>(p.ws) : p.out_f32;   // one range: its partial sums are the result
     int64_t max_tasks;
     if (p.experts == nullptr) {
         a.dense_tasks = static_cast<int>((p.rows + max_tok - 1) / max_tok);
@@ -715,12 +720,13 @@ static int run_problem(const Problem& p, cudaStream_t stream) {
                 (long long)(grid * cg), (long long)(max_tasks * mtiles));
     rc = dispatch_gemm(p.qt, p.mode, cg, wide ? 1 : 0, a, static_cast<int>(grid * cg), stream);
     if (rc != TGO_OK) return rc;
-    if (nsplit > 1) {
+    if (a.partial != nullptr) {
         const long long n_vec = p.rows * p.K / 4;   // K is a multiple of 256
         long long blocks = (n_vec + 255) / 256;
         if (blocks > num_sms() * 8LL) blocks = num_sms() * 8LL;
-        split_reduce_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(static_cast<const float4*>(p.ws), nsplit, n_vec,
-                                                                          static_cast<uint2*>(p.out[0]));
+        split_reduce_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(reinterpret_cast<const float4*>(a.partial), nsplit, n_vec,
+                                                                          static_cast<uint2*>(p.out[0]),
+                                                                          nsplit > 1 ? reinterpret_cast<float4*>(p.out_f32) : nullptr);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "split_reduce_kernel launch");
     }
@@ -879,6 +885,23 @@ int tgo_mmq_dx_ws(const void* dy, const void* packed_weight, void* dx, int64_t r
     p.ws = workspace; p.ws_bytes = workspace_bytes;
     return run_problem(p, static_cast<cudaStream_t>(stream));
 }
+
+}  // extern "C"
+
+namespace tgo {
+// tgo_mmq_dx_ws that also writes the result before its rounding to dx_f32 (16-byte aligned, may be null).
+int mmq_dx_f32(const void* dy, const void* packed_weight, void* dx, float* dx_f32, int64_t rows, int64_t out_features,
+               int64_t in_features, int quant_type, void* workspace, int64_t workspace_bytes, void* stream) {
+    if (dx_f32 != nullptr && !aligned16(dx_f32)) return fail(TGO_E_ARG, "output data pointer must be 16-byte aligned");
+    Problem p = {};
+    p.act[0] = dy; p.wgt[0] = packed_weight; p.out[0] = dx; p.nsets = 1;
+    p.rows = rows; p.N = out_features; p.K = in_features; p.E = 1; p.qt = quant_type; p.mode = kBwd;
+    p.ws = workspace; p.ws_bytes = workspace_bytes; p.out_f32 = dx_f32;
+    return run_problem(p, static_cast<cudaStream_t>(stream));
+}
+}  // namespace tgo
+
+extern "C" {
 
 int tgo_mmq_fwd_multi(const void* x, const void* const* packed_weights, void* const* ys, int64_t num_weights, int64_t rows,
                       int64_t out_features, int64_t in_features, int quant_type, void* stream) {

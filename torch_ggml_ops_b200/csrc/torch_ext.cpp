@@ -15,6 +15,8 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 
+#include <cmath>
+
 #include "../../include/tgo_mmq.h"
 
 namespace {
@@ -342,8 +344,9 @@ std::tuple<Tensor, Tensor> swiglu_grad_autograd(const Tensor& d, const Tensor& g
 }
 
 // ------------------------------------------------------------------ lm_head_loss
-std::tuple<Tensor, Tensor> lm_head_cuda(const Tensor& hidden, const Tensor& w, int64_t qt, int64_t vocab, const Tensor& targets, int64_t chunk_rows,
-                                        double grad_scale) {
+// loss, d_hidden and, if asked for, d_hidden before its rounding
+std::tuple<Tensor, Tensor, Tensor> lm_head_run(const Tensor& hidden, const Tensor& w, int64_t qt, int64_t vocab, const Tensor& targets,
+                                               int64_t chunk_rows, double grad_scale, bool want_f32) {
     TORCH_CHECK(hidden.is_cuda(), "input must be a CUDA tensor");
     TORCH_CHECK(hidden.scalar_type() == at::kBFloat16, "input must have dtype torch.bfloat16");
     TORCH_CHECK(hidden.dim() == 2, "hidden must have shape [rows, in_features]");
@@ -363,29 +366,45 @@ std::tuple<Tensor, Tensor> lm_head_cuda(const Tensor& hidden, const Tensor& w, i
     if (reinterpret_cast<uintptr_t>(x.const_data_ptr()) % 16 != 0) x = x.clone();
     const c10::cuda::CUDAGuard guard(x.device());
     Tensor d_hidden = at::empty({rows, k}, x.options());
-    if (rows == 0) return {at::zeros({}, x.options().dtype(at::kFloat)), d_hidden};
+    Tensor d_f32 = want_f32 ? at::empty({rows, k}, x.options().dtype(at::kFloat)) : Tensor();
+    if (rows == 0) return {at::zeros({}, x.options().dtype(at::kFloat)), d_hidden, d_f32};
     Tensor loss = at::empty({}, x.options().dtype(at::kFloat));
     const int64_t bytes = tgo_lm_head_loss_workspace_bytes(rows, vocab, k, static_cast<int>(qt), chunk_rows);
     TORCH_CHECK(bytes >= 0, "chunk_rows must be positive");
     Tensor ws = at::empty({bytes}, x.options().dtype(at::kByte));
-    check_rc(tgo_lm_head_loss(x.const_data_ptr(), w.const_data_ptr(), targets.const_data_ptr<int64_t>(), rows, vocab, k, static_cast<int>(qt),
-                              chunk_rows, static_cast<float>(grad_scale), loss.mutable_data_ptr<float>(), d_hidden.mutable_data_ptr(),
-                              ws.mutable_data_ptr(), bytes, stream_of(x)),
+    check_rc(tgo_lm_head_loss_f32(x.const_data_ptr(), w.const_data_ptr(), targets.const_data_ptr<int64_t>(), rows, vocab, k, static_cast<int>(qt),
+                                  chunk_rows, static_cast<float>(grad_scale), loss.mutable_data_ptr<float>(), d_hidden.mutable_data_ptr(),
+                                  want_f32 ? d_f32.mutable_data_ptr<float>() : nullptr, ws.mutable_data_ptr(), bytes, stream_of(x)),
              "lm_head_loss");
-    return {loss, d_hidden};
+    return {loss, d_hidden, d_f32};
+}
+std::tuple<Tensor, Tensor> lm_head_cuda(const Tensor& hidden, const Tensor& w, int64_t qt, int64_t vocab, const Tensor& targets, int64_t chunk_rows,
+                                        double grad_scale) {
+    auto [loss, d, f] = lm_head_run(hidden, w, qt, vocab, targets, chunk_rows, grad_scale, false);
+    return {loss, d};
+}
+std::tuple<Tensor, Tensor, Tensor> lm_head_f32_cuda(const Tensor& hidden, const Tensor& w, int64_t qt, int64_t vocab, const Tensor& targets,
+                                                    int64_t chunk_rows, double grad_scale) {
+    return lm_head_run(hidden, w, qt, vocab, targets, chunk_rows, grad_scale, true);
 }
 std::tuple<Tensor, Tensor> call_lm_head(const Tensor& x, const Tensor& w, int64_t qt, int64_t vocab, const Tensor& t, int64_t chunk, double scale) {
     static const auto h = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, int64_t, int64_t, const Tensor&, int64_t, double)>(
         "torch_ggml_ops_b200::lm_head_loss");
     return h.call(x, w, qt, vocab, t, chunk, scale);
 }
+std::tuple<Tensor, Tensor, Tensor> call_lm_head_f32(const Tensor& x, const Tensor& w, int64_t qt, int64_t vocab, const Tensor& t, int64_t chunk,
+                                                    double scale) {
+    static const auto h = op<std::tuple<Tensor, Tensor, Tensor>(const Tensor&, const Tensor&, int64_t, int64_t, const Tensor&, int64_t, double)>(
+        "torch_ggml_ops_b200::lm_head_loss_f32");
+    return h.call(x, w, qt, vocab, t, chunk, scale);
+}
 [[noreturn]] void no_second_order_head() { TORCH_CHECK(false, "torch_ggml_ops_b200::lm_head_loss does not support higher-order gradients"); }
-// d * g * scale, the gradient that autograd gets.  The loss is not linear in hidden and d has no graph, so
+// d * g * scale, the gradient that autograd gets: d in fp32, so that the product is rounded once.  The loss is not linear in hidden and d has no graph, so
 // a second derivative is refused; `edge` ties the result to hidden for that.
 struct LmHeadGradFn : public Function<LmHeadGradFn> {
     static Tensor forward(AutogradContext*, const Tensor& edge, const Tensor& d, const Tensor& g, double scale) {
         at::AutoDispatchBelowADInplaceOrView guard;
-        return (d.to(at::kFloat) * (g * scale)).to(d.scalar_type());
+        return (d * (g * scale)).to(edge.scalar_type());
     }
     static tensor_list backward(AutogradContext*, tensor_list) { no_second_order_head(); }
 };
@@ -395,10 +414,12 @@ struct LmHeadFn : public Function<LmHeadFn> {
     static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& edge, const Tensor& w, int64_t qt, int64_t vocab,
                                  const Tensor& t, int64_t chunk, double scale) {
         at::AutoDispatchBelowADInplaceOrView guard;
-        auto [loss, d] = call_lm_head(x, w, qt, vocab, t, chunk, scale);
-        Tensor unscaled = scale != 0.0 ? d : std::get<1>(call_lm_head(x, w, qt, vocab, t, chunk, 1.0));
+        // a scale that could be divided out again without leaving bf16's range serves both
+        const bool serves = std::abs(scale) >= 0x1p-40 && std::abs(scale) <= 0x1p40;
+        auto [loss, d, unscaled] = call_lm_head_f32(x, w, qt, vocab, t, chunk, scale);
+        if (!serves) unscaled = std::get<2>(call_lm_head_f32(x, w, qt, vocab, t, chunk, 1.0));
         ctx->save_for_backward({unscaled, edge});
-        ctx->saved_data["scale"] = scale != 0.0 ? 1.0 / scale : 1.0;
+        ctx->saved_data["scale"] = serves ? 1.0 / scale : 1.0;
         ctx->set_materialize_grads(false);
         return {loss, d};
     }
@@ -440,12 +461,16 @@ TORCH_LIBRARY_FRAGMENT(torch_ggml_ops_b200, m) {
     m.def(
         "lm_head_loss(Tensor hidden, Tensor packed_weight, int quant_type, int vocab, Tensor targets, int chunk_rows, float grad_scale) -> "
         "(Tensor, Tensor)");
+    m.def(
+        "lm_head_loss_f32(Tensor hidden, Tensor packed_weight, int quant_type, int vocab, Tensor targets, int chunk_rows, float grad_scale) -> "
+        "(Tensor, Tensor, Tensor)");
 }
 TORCH_LIBRARY_IMPL(torch_ggml_ops_b200, CUDA, m) {
     m.impl("mmq_multi", &multi_cuda);
     m.impl("swiglu", &swiglu_cuda);
     m.impl("swiglu_grad", &swiglu_grad_cuda);
     m.impl("lm_head_loss", &lm_head_cuda);
+    m.impl("lm_head_loss_f32", &lm_head_f32_cuda);
 }
 TORCH_LIBRARY_IMPL(torch_ggml_ops_b200, Autograd, m) {
     m.impl("mmq_multi", &multi_autograd);

@@ -41,6 +41,11 @@ def _(hidden, packed_weight, quant_type, vocab, targets, chunk_rows, grad_scale)
     return hidden.new_empty((), dtype=torch.float32), torch.empty_like(hidden)
 
 
+@torch.library.register_fake(f"{_NS}::lm_head_loss_f32")   # with the gradient before its rounding, for autograd
+def _(hidden, packed_weight, quant_type, vocab, targets, chunk_rows, grad_scale):
+    return hidden.new_empty((), dtype=torch.float32), torch.empty_like(hidden), hidden.new_empty(hidden.shape, dtype=torch.float32)
+
+
 def mmq_multi(input: torch.Tensor, packed_weights, quant_type: int, out_features: int):
     """``[input @ W_i.T for W_i in packed_weights]`` (1 to 4 weights of one quant type and shape
     [out_features, in_features]) with two weight sets per kernel launch; every result is

@@ -30,6 +30,7 @@ SIGNATURES = {
     "tgo_mmq_fwd_multi": (_i32, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _i32, _vp]),
     "tgo_lm_head_loss_workspace_bytes": (_i64, [_i64, _i64, _i64, _i32, _i64]),
     "tgo_lm_head_loss": (_i32, [_vp, _vp, _vp, _i64, _i64, _i64, _i32, _i64, ctypes.c_float, _vp, _vp, _vp, _i64, _vp]),
+    "tgo_lm_head_loss_f32": (_i32, [_vp, _vp, _vp, _i64, _i64, _i64, _i32, _i64, ctypes.c_float, _vp, _vp, _vp, _vp, _i64, _vp]),
     "tgo_grouped_workspace_bytes": (_i64, [_i64, _i64]),
     "tgo_build_tiles": (_i32, [_vp, _vp, _i64, _i64, _i64, _i64, _vp, _i64, _vp]),
     "tgo_grouped_fwd": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _i64, _vp]),
