@@ -42,5 +42,36 @@ def test_gradient_through_autograd(cuda, name, qt, V, K, T, chunk):
         (out * cotangent).backward()
         assert torch.equal(x.grad, (d32 * cotangent).to(torch.bfloat16))   # powers of two: the scale leaves no trace
         assert ref.rel_frobenius(x.grad.double().cpu(), want * cotangent) < 1e-2
-        assert abs(float(out) - float(want_loss)) < 2e-3 * float(want_loss)
+        assert abs(float(out.detach()) - float(want_loss)) < 2e-3 * float(want_loss)
         assert ref.rel_frobenius(dh.detach().double().cpu(), want * scale) < 1e-2 if scale else not dh.detach().any()
+
+
+def _q6_rows(d):
+    """Q6_K rows of one block whose 256 weights are all d (quants 33 - 32, scales 1), d a list of fp16 values."""
+    b = np.zeros((len(d), 210), dtype=np.uint8)
+    b[:, :128], b[:, 128:192], b[:, 192:208] = 0x11, 0xAA, 1
+    b[:, 208:] = np.asarray(d, dtype=np.float16).view(np.uint8).reshape(-1, 2)
+    return b
+
+
+@pytest.mark.parametrize("at", [0, 8, 504, 992])
+@pytest.mark.parametrize("bad", [[np.nan] * 8, [np.inf] * 7 + [np.nan], [np.inf] * 8, [-np.inf] * 8])
+def test_non_finite_logits(cuda, bad, at):
+    """x = -1: eight neighbouring columns are NaN, -inf or +inf, those that one thread of the statistics reads
+    first among them; loss and gradient as log_softmax defines them."""
+    import torch_ggml_ops_b200 as tgo
+
+    V, K, T = 1000, 256, 40
+    w, W, _ = dense_case(ref.Q6_K, V, K, 3)
+    w = w.reshape(V, 210).copy()
+    w[at:at + 8] = _q6_rows(bad)
+    targets = torch.full((T,), 20)
+    x = torch.full((T, K), -1.0, dtype=torch.bfloat16)
+    logits = (x.double() @ torch.from_numpy(W).double().t())
+    logits[:, at:at + 8] = -torch.tensor(bad, dtype=torch.float64)
+    want = torch.nn.functional.cross_entropy(logits, targets, reduction="sum")
+    loss, dh = tgo.lm_head_loss(to_dev(x), to_dev(w), ref.Q6_K, V, to_dev(targets))
+    if torch.isnan(want):
+        assert torch.isnan(loss) and torch.isnan(dh).all()
+    else:   # the columns have no probability; 0 * inf leaves no gradient
+        assert abs(float(loss) - float(want)) < 2e-3 * abs(float(want))

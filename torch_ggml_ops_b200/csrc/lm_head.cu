@@ -78,10 +78,11 @@ __global__ void __launch_bounds__(kXentThreads) xent_stats_kernel(const __nv_bfl
             acc.s *= __expf(acc.m - m);   // acc.m = -inf at first: 0 * 0
             acc.m = m;
         }
-        if (acc.m == -INFINITY) continue;   // nothing but -inf so far: they add nothing
+        // nothing but -inf so far (they add exp(-inf) = 0) and NaN (which no maximum shows, but the sum does)
+        const float base = acc.m == -INFINITY ? 0.0f : acc.m;
         float s = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) s += __expf(f[j] - acc.m);
+        for (int j = 0; j < 8; ++j) s += __expf(f[j] - base);
         acc.s += s;
     }
     __shared__ MaxSum warp_part[kXentThreads / 32];
