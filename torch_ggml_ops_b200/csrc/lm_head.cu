@@ -27,7 +27,7 @@ struct MaxSum {
 };
 __device__ __forceinline__ MaxSum merge(MaxSum a, MaxSum b) {
     const float m = fmaxf(a.m, b.m);   // an empty part has m = -inf, s = 0
-    return {m, (a.m == m ? a.s : a.s * __expf(a.m - m)) + (b.m == m ? b.s : b.s * __expf(b.m - m))};
+    return {m, (a.m == m ? a.s : a.s * expf(a.m - m)) + (b.m == m ? b.s : b.s * expf(b.m - m))};
 }
 
 // Elements of a row as 16-byte vectors: the first `head` ones and those after the last vector are
@@ -75,14 +75,14 @@ __global__ void __launch_bounds__(kXentThreads) xent_stats_kernel(const __nv_bfl
 #pragma unroll
         for (int j = 1; j < 8; ++j) m = fmaxf(m, f[j]);
         if (m > acc.m) {
-            acc.s *= __expf(acc.m - m);   // acc.m = -inf at first: 0 * 0
+            acc.s *= expf(acc.m - m);   // acc.m = -inf at first: 0 * 0
             acc.m = m;
         }
         // nothing but -inf so far (they add exp(-inf) = 0) and NaN (which no maximum shows, but the sum does)
         const float base = acc.m == -INFINITY ? 0.0f : acc.m;
         float s = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) s += __expf(f[j] - base);
+        for (int j = 0; j < 8; ++j) s += expf(f[j] - base);
         acc.s += s;
     }
     __shared__ MaxSum warp_part[kXentThreads / 32];
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kXentThreads) xent_grad_kernel(__nv_bfloat16* 
     for (int i = 1; i < static_cast<int>(gridDim.x); ++i) all = merge(all, part[row * gridDim.x + i]);
     const float lse = all.m + logf(all.s);
     const long long target = targets[row];
-    auto grad = [&](float v, long long col) { return (__expf(v - lse) - (col == target ? 1.0f : 0.0f)) * scale; };
+    auto grad = [&](float v, long long col) { return (expf(v - lse) - (col == target ? 1.0f : 0.0f)) * scale; };
     if (blockIdx.x == 0) {
         if (threadIdx.x == 0) row_loss[row] = lse - target_logit[row];
         if (threadIdx.x < r.head) x[threadIdx.x] = __float2bfloat16(grad(__bfloat162float(x[threadIdx.x]), threadIdx.x));
@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(kXentThreads) xent_grad_kernel(__nv_bfloat16* 
         float p[8];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            p[2 * j] = __expf(__uint_as_float(w[j] << 16) - lse) * scale;
-            p[2 * j + 1] = __expf(__uint_as_float(w[j] & 0xFFFF0000u) - lse) * scale;
+            p[2 * j] = expf(__uint_as_float(w[j] << 16) - lse) * scale;
+            p[2 * j + 1] = expf(__uint_as_float(w[j] & 0xFFFF0000u) - lse) * scale;
         }
         if (static_cast<unsigned long long>(target - col) < 8ull) {
 #pragma unroll
