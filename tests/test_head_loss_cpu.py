@@ -83,3 +83,13 @@ def test_the_gradient_is_rounded_once(head, grad_scale):
         (torch.nn.functional.cross_entropy(y @ w.double().t(), targets, reduction="sum") * cotangent).backward()
         unit = torch.exp2(torch.floor(torch.log2(y.grad.abs())) - 7)
         assert bool(((x.grad.double() - y.grad).abs() <= 0.501 * unit + 1e-6 * y.grad.abs().max()).all())
+
+
+def test_no_rows(head):
+    """Nothing to compute: a loss of zero and an empty gradient, whatever the weight and the device."""
+    import torch_ggml_ops_b200 as tgo
+
+    for hidden in (torch.empty(0, K, dtype=torch.bfloat16), torch.empty(2, 0, K), torch.empty(0, K, dtype=torch.bfloat16, requires_grad=True)):
+        loss, d = tgo.lm_head_loss(hidden, torch.empty(0, dtype=torch.uint8), 14, V, torch.empty(0, dtype=torch.long))
+        assert loss.dtype == torch.float32 and float(loss) == 0.0 and not loss.requires_grad
+        assert d.shape == hidden.shape and d.dtype == hidden.dtype

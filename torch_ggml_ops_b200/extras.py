@@ -86,6 +86,8 @@ def lm_head_loss(hidden: torch.Tensor, packed_weight: torch.Tensor, quant_type: 
     t1 = targets.reshape(-1)
     if t1.numel() != h2.shape[0]:
         raise ValueError("targets must have one entry per row of hidden")
+    if h2.shape[0] == 0:
+        return torch.zeros((), dtype=torch.float32, device=hidden.device), torch.empty_like(h2).reshape(hidden.shape)
     loss, d_hidden = _ops.lm_head_loss.default(h2, packed_weight, int(quant_type), int(vocab), t1.long().contiguous(), int(chunk_rows),
                                                float(grad_scale))
     return loss, d_hidden.reshape(hidden.shape)
