@@ -75,3 +75,24 @@ def test_non_finite_logits(cuda, bad, at):
         assert torch.isnan(loss) and torch.isnan(dh).all()
     else:   # the columns have no probability; 0 * inf leaves no gradient
         assert abs(float(loss) - float(want)) < 2e-3 * abs(float(want))
+
+
+def test_strided_hidden(cuda):
+    """Rows that lie apart are taken, columns that do are refused; the gradient has the layout that the fake
+    kernel promises."""
+    import torch_ggml_ops_b200 as tgo
+
+    qt, V, K, T = ref.Q6_K, 1000, 256, 50
+    w, _, hidden, targets = _inputs(qt, V, K, T)
+    wd, td = to_dev(w), to_dev(targets)
+    padded = to_dev(torch.nn.functional.pad(hidden, (3, 5)))[:, 3:3 + K]
+    across = to_dev(hidden.t().contiguous()).t()
+    for x, chunk in ((padded, 256), (padded, 16), (across, 1)):
+        compiled = torch.compile(lambda h: tgo.lm_head_loss(h, wd, qt, V, td, chunk_rows=chunk), backend="aot_eager", fullgraph=True)
+        loss, d = tgo.lm_head_loss(to_dev(hidden), wd, qt, V, td, chunk_rows=chunk)
+        for got_loss, got in (tgo.lm_head_loss(x, wd, qt, V, td, chunk_rows=chunk), compiled(x)):
+            assert got.stride() == torch.empty_like(x).stride()
+            assert torch.equal(got, d) and torch.equal(got_loss, loss)
+    for chunk in (256, 20, 49):
+        with pytest.raises(RuntimeError, match="contiguous"):
+            tgo.lm_head_loss(across, wd, qt, V, td, chunk_rows=chunk)

@@ -15,6 +15,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "../../include/tgo_mmq.h"
@@ -362,21 +363,31 @@ std::tuple<Tensor, Tensor, Tensor> lm_head_run(const Tensor& hidden, const Tenso
     TORCH_CHECK(vocab > 0, "out_features must be positive; got ", vocab);
     const int64_t expected = vocab * (k / 256) * block_bytes(qt);
     TORCH_CHECK(w.numel() == expected, "packed_weight has ", w.numel(), " bytes, expected ", expected, " for [", vocab, ", ", k, "] quant_type=", qt);
+    TORCH_CHECK(chunk_rows > 0, "chunk_rows must be positive");
+    if (!hidden.is_contiguous() && rows > 0) {
+        // a chunk is copied where it is a view, and a copy keeps the order of the strides: rows may lie apart, columns not
+        const int64_t chunk = std::min(chunk_rows, rows), last = rows % chunk;
+        for (const int64_t n : {chunk, last > 0 ? last : chunk})
+            TORCH_CHECK(at::empty_like(hidden.narrow(0, 0, n), hidden.options().device(at::kMeta)).is_contiguous(),
+                        "input must be contiguous; torch_ggml_ops will not insert a hidden copy");
+    }
+    const c10::cuda::CUDAGuard guard(hidden.device());
     Tensor x = hidden.contiguous();
     if (reinterpret_cast<uintptr_t>(x.const_data_ptr()) % 16 != 0) x = x.clone();
-    const c10::cuda::CUDAGuard guard(x.device());
-    Tensor d_hidden = at::empty({rows, k}, x.options());
+    Tensor like_hidden = at::empty_like(hidden);
+    Tensor d_hidden = like_hidden.is_contiguous() ? like_hidden : at::empty({rows, k}, x.options());
     Tensor d_f32 = want_f32 ? at::empty({rows, k}, x.options().dtype(at::kFloat)) : Tensor();
-    if (rows == 0) return {at::zeros({}, x.options().dtype(at::kFloat)), d_hidden, d_f32};
+    if (rows == 0) return {at::zeros({}, x.options().dtype(at::kFloat)), like_hidden, d_f32};
     Tensor loss = at::empty({}, x.options().dtype(at::kFloat));
     const int64_t bytes = tgo_lm_head_loss_workspace_bytes(rows, vocab, k, static_cast<int>(qt), chunk_rows);
-    TORCH_CHECK(bytes >= 0, "chunk_rows must be positive");
+    TORCH_CHECK(bytes >= 0, "unsupported sizes");
     Tensor ws = at::empty({bytes}, x.options().dtype(at::kByte));
     check_rc(tgo_lm_head_loss_f32(x.const_data_ptr(), w.const_data_ptr(), targets.const_data_ptr<int64_t>(), rows, vocab, k, static_cast<int>(qt),
                                   chunk_rows, static_cast<float>(grad_scale), loss.mutable_data_ptr<float>(), d_hidden.mutable_data_ptr(),
                                   want_f32 ? d_f32.mutable_data_ptr<float>() : nullptr, ws.mutable_data_ptr(), bytes, stream_of(x)),
              "lm_head_loss");
-    return {loss, d_hidden, d_f32};
+    if (!like_hidden.is_contiguous()) like_hidden.copy_(d_hidden);
+    return {loss, like_hidden, d_f32};
 }
 std::tuple<Tensor, Tensor> lm_head_cuda(const Tensor& hidden, const Tensor& w, int64_t qt, int64_t vocab, const Tensor& targets, int64_t chunk_rows,
                                         double grad_scale) {
