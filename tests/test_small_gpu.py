@@ -62,3 +62,62 @@ def test_several_weights_in_one_launch(cuda):
     x = to_dev(blocks.gaussian_bf16((M, K), 9))
     for y, w in zip(tgo.mmq_multi(x, ws, qt, N), ws):
         assert torch.equal(y, tgo.mmq(x, w, qt, N))
+
+
+@pytest.mark.parametrize("name,qt", ALL_TYPES)
+@pytest.mark.parametrize("M,N,K", [(3, 17, 512), (17, 72, 2304), (24, 200, 512)])
+def test_infinite_and_huge_values(cuda, name, qt, M, N, K):
+    """An infinite activation gives the infinities of the weights' signs (NaN where two meet or the weight is
+    zero), a huge one the finite product, an infinite block scale likewise; other tokens and rows keep their bits."""
+    import torch_ggml_ops_b200 as tgo
+
+    w, W, Wb = dense_case(qt, N, K, 3 + qt)
+    x = blocks.gaussian_bf16((M, K), M)
+    plain = tgo.mmq(to_dev(x), to_dev(w), qt, N).cpu()
+    odd = x.clone()
+    odd[0, K - 1] = float("inf")
+    odd[1, 5], odd[1, 300] = float("-inf"), float("inf")
+    odd[2] *= 2.0 ** 118
+    bad = np.asarray(w).reshape(N, K // 256, -1).copy()
+    d_at = {ref.Q3_K: 108, ref.Q6_K: 208}.get(qt, 0)
+    bad[5, 1, d_at:d_at + 2] = np.array([np.inf], dtype=np.float16).view(np.uint8)
+    Wd = Wb.double()
+    y = tgo.mmq(to_dev(odd), to_dev(w), qt, N).cpu()
+    want = (odd.double()[:3, None, :] * Wd[None]).sum(-1)
+    assert torch.equal(torch.isnan(y[:2]), torch.isnan(want[:2]))
+    live = ~torch.isnan(want[:2])
+    assert torch.equal(y[:2].double()[live], want[:2][live]) and bool(torch.isinf(want[:2][live]).all())
+    assert bool(torch.isfinite(y[2]).all()) and ref.rel_frobenius(y[2].double() * 2.0 ** -118, want[2] * 2.0 ** -118) < 2.0 ** -7
+    assert torch.equal(y[3:], plain[3:])
+    # one infinite scale: that row alone, infinite or NaN as the decoded weights make it
+    z = tgo.mmq(to_dev(x), to_dev(bad), qt, N).cpu()
+    wide = tgo.mmq(to_dev(torch.cat([x, x.new_zeros(64, K)])), to_dev(bad), qt, N).cpu()[:M]   # enough rows for the tile GEMM
+    assert bool((~torch.isfinite(z[:, 5])).all())
+    assert torch.equal(torch.isnan(z[:, 5]), torch.isnan(wide[:, 5])) and torch.equal(torch.nan_to_num(z[:, 5]), torch.nan_to_num(wide[:, 5]))
+    keep = torch.arange(N) != 5
+    assert torch.equal(z[:, keep], plain[:, keep])
+
+
+@pytest.mark.parametrize("name,qt", ALL_TYPES)
+def test_infinite_values_in_groups(cuda, name, qt):
+    from torch_ggml_ops_b200 import native
+
+    sizes, ids, E, N, K = [3, 9, 1, 12], [4, 1, 3, 0], 5, 40, 512
+    w0, w1 = (blocks.expert_weights(qt, E, N, K, s) for s in (1, 2))
+    ei, eo = routing_from_sizes(sizes, ids)
+    R = sum(sizes)
+    x = blocks.gaussian_bf16((R, K), 3)
+    x[4, 17], x[20, 511] = float("inf"), float("-inf")
+    y0, y1 = (torch.empty((R, N), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    ws = torch.empty(native.grouped_workspace_bytes(R, len(sizes)), dtype=torch.uint8, device="cuda")
+    native.grouped_fwd(to_dev(x), to_dev(w0), to_dev(w1), y0, y1, to_dev(ei), to_dev(eo), E, R, N, K, qt, ws)
+    for y, w in ((y0, w0), (y1, w1)):
+        got = y.double().cpu()
+        W = torch.from_numpy(ref.expert_weights_fp32(w, qt, N, K)).to(torch.bfloat16).double()
+        for r, e in ((4, 1), (20, 0)):
+            want = (x[r].double() * W[e]).sum(-1)
+            assert torch.equal(torch.isnan(got[r]), torch.isnan(want))
+            assert torch.equal(got[r][~torch.isnan(want)], want[~torch.isnan(want)])
+        rest = torch.ones(R, dtype=torch.bool)
+        rest[[4, 20]] = False
+        assert bool(torch.isfinite(got[rest]).all())

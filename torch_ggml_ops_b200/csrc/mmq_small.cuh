@@ -27,6 +27,10 @@
 // * Persistent CTAs take contiguous ranges of the (token tile, weight set, row tile) units, so the
 //   activation fragments are rebuilt only where the token tile changes.  Grouped calls find their
 //   token tiles by a prefix sum over the groups in every CTA: no tile list, no second launch.
+// * The bias and the group sums take an infinite activation or block scale to inf - inf, and leave
+//   fp32's range before the product does (from |x| of some 1e36, 1e26 with the largest scales).  Both
+//   show as a sum that is not finite, and such sums alone are computed again from decoded weights, as
+//   the GEMM does; nothing of that is in the loop over the blocks.
 #pragma once
 
 #include "gguf_decode.cuh"
@@ -436,6 +440,154 @@ __device__ __forceinline__ int small_scan_groups(const SmallArgs& a, int tok, in
     return base;
 }
 
+// `cum`: the three lists of small_scan_groups, one after the other
+__device__ __forceinline__ SmallTile small_tile_at(const SmallArgs& a, int tok, const int* cum, int tile) {
+    SmallTile r;
+    if (a.experts == nullptr) {
+        r.expert = 0;
+        r.row0 = tile * tok;
+        r.ntok = min(tok, a.rows - r.row0);
+        return r;
+    }
+    int lo = 0, hi = a.groups - 1;   // first group whose cumulative count exceeds the tile
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (cum[mid] > tile) hi = mid; else lo = mid + 1;
+    }
+    const int first = lo > 0 ? cum[lo - 1] : 0;
+    r.expert = cum[2 * a.groups + lo];
+    r.row0 = cum[a.groups + lo] + (tile - first) * tok;
+    r.ntok = min(tok, a.offsets[lo] - r.row0);
+    return r;
+}
+
+// A CTA's range of the (token tile, weight set, group of rw row tiles) units; a unit's coordinates
+// advance by carries, without divisions.
+struct SmallWalk {
+    struct Unit {
+        int u, tile, set, rg;
+    };
+    int rtg, lo, hi;
+    __device__ __forceinline__ SmallWalk(const SmallArgs& a, int ntiles) {
+        rtg = (a.out_features + 16 * a.rw - 1) / (16 * a.rw);   // row-tile groups of a weight set
+        const long long units = static_cast<long long>(ntiles) * rtg * a.nsets;
+        lo = static_cast<int>(units * blockIdx.x / gridDim.x);
+        hi = static_cast<int>(units * (blockIdx.x + 1) / gridDim.x);
+    }
+    __device__ __forceinline__ Unit first(const SmallArgs& a) const {
+        Unit w;
+        w.u = lo;
+        w.tile = lo / (rtg * a.nsets);
+        w.set = (lo - w.tile * rtg * a.nsets) / rtg;
+        w.rg = lo - (w.tile * a.nsets + w.set) * rtg;
+        return w;
+    }
+    __device__ __forceinline__ void advance(const SmallArgs& a, Unit& w) const {
+        ++w.u;
+        if (++w.rg == rtg) {
+            w.rg = 0;
+            if (++w.set == a.nsets) { w.set = 0; ++w.tile; }
+        }
+    }
+};
+
+// 16 weight rows x 8 tokens as the GEMM computes them: weights decoded to bf16, times x, summed in fp32.
+//   off: byte of the first row in the tensor; last: its last row that exists (0..15); x: the first of ntok tokens
+//   stage: a stage of this warp, none in flight; v: the elements of this thread's mma fragment
+template <int QT>
+__device__ __forceinline__ void small_direct(const uint8_t* wgt, long long wgt_bytes, long long off, int row_bytes, int last, int nkb,
+                                          const __nv_bfloat16* x, int ntok, uint32_t stage, uint32_t grid, float (&v)[4]) {
+    using Fmt = BlockFmt<QT>;
+    using Sf = SmallFmt<QT>;
+    const int lane = threadIdx.x & 31, row = lane & 15, half = lane >> 4, K = nkb * 256;
+    float acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+    for (int kb = 0; kb < nkb; ++kb) {
+        __syncwarp();
+        for (int c = lane; c < 16 * Sf::kChunks; c += 32) {
+            const int r = c / Sf::kChunks, po = (c - r * Sf::kChunks) * 16;
+            const long long at = ((off + static_cast<long long>(min(r, last)) * row_bytes + kb * Fmt::kBytes) & ~15LL) + po;
+            const int n = static_cast<int>(max(0LL, min(16LL, wgt_bytes - at)));
+            cp_async16(stage + r * Sf::kPitch + po, n > 0 ? wgt + at : wgt, n);
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncwarp();
+        const long long at = off + static_cast<long long>(min(row, last)) * row_bytes + kb * Fmt::kBytes;
+        const uint32_t blk = stage + row * Sf::kPitch + static_cast<uint32_t>(at & 15);
+#pragma unroll 1
+        for (int g = 4 * half; g < 4 * half + 4; ++g) {
+            uint4 w[4];
+            decode32<QT>(blk, g, grid, w);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (j >= ntok) break;
+                const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<long long>(j) * K + kb * 256 + g * 32);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const uint4 xs = src[c];
+                    const uint32_t a[4] = {w[c].x, w[c].y, w[c].z, w[c].w}, b[4] = {xs.x, xs.y, xs.z, xs.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 wf = __bfloat1622float2(as_bf162(a[i])), xf = __bfloat1622float2(as_bf162(b[i]));
+                        acc[j] = fmaf(wf.x, xf.x, acc[j]);
+                        acc[j] = fmaf(wf.y, xf.y, acc[j]);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float sum = acc[j] + __shfl_xor_sync(0xFFFFFFFFu, acc[j], 16);
+        const float lo = __shfl_sync(0xFFFFFFFFu, sum, lane >> 2), hi = __shfl_sync(0xFFFFFFFFu, sum, (lane >> 2) + 8);
+        if ((j >> 1) == (lane & 3)) { v[j & 1] = lo; v[2 + (j & 1)] = hi; }
+    }
+}
+__device__ __forceinline__ bool not_finite(float v) { return (__float_as_uint(v) & 0x7F800000u) == 0x7F800000u; }
+
+// After the kernel's walk: every thread looks again at the results that it stored and replaces those
+// that are not finite.  A function of its own, so that the kernel keeps no register for it.
+template <int QT, int NT>
+__device__ __noinline__ void small_redo(const SmallArgs& args, int ntiles, const int* cum, uint32_t my_ring, uint32_t grid_s) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int kw = args.kw, rw = args.rw, rwi = warp / kw, ks = warp - rwi * kw;
+    const int N = args.out_features, K = args.in_features;
+    const SmallWalk walk(args, ntiles);
+    int turn = 0;   // as in the kernel: the thread that stored a result reads it back
+    for (SmallWalk::Unit un = walk.first(args); un.u < walk.hi; walk.advance(args, un)) {
+        const SmallTile ct = small_tile_at(args, 8 * NT, cum, un.tile);
+        const int row0 = (un.rg * rw + rwi) * 16;
+        for (int nt = 0; nt < NT; ++nt) {
+            const bool mine = ks == turn;
+            if (++turn == kw) turn = 0;
+            if (!mine || nt * 8 >= ct.ntok || row0 >= N) continue;
+            __nv_bfloat16* at[4];
+            bool redo[4], any = false;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int token = nt * 8 + 2 * t + (j & 1), row = row0 + g + 8 * (j >> 1), r = ct.row0 + token;
+                at[j] = nullptr;
+                if (token < ct.ntok && row < N) {
+                    at[j] = args.out_rows != nullptr ? args.out_rows[r] : args.out[un.set] + static_cast<long long>(r) * N;
+                    if (at[j] != nullptr) at[j] += row;
+                }
+                redo[j] = at[j] != nullptr && not_finite(__bfloat162float(*at[j]));
+                any |= redo[j];
+            }
+            if (!__any_sync(0xFFFFFFFFu, any)) continue;
+            float v[4];
+            small_direct<QT>(args.wgt[un.set], args.wgt_bytes, (static_cast<long long>(ct.expert) * N + row0) * args.row_bytes, args.row_bytes,
+                             min(15, N - 1 - row0), K >> 8, args.act + static_cast<long long>(ct.row0 + nt * 8) * K, ct.ntok - nt * 8, my_ring,
+                             grid_s, v);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (redo[j]) *at[j] = __float2bfloat16(v[j]);
+        }
+    }
+}
+
 template <int QT, int NT>
 __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __grid_constant__ SmallArgs args) {
     using Fmt = BlockFmt<QT>;
@@ -456,51 +608,18 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
     const uint32_t red_s = ring_s + nwarps * S * Sf::kStageBytes;
     int* const lists = reinterpret_cast<int*>(smem + (red_s - frag_s) + (kw > 1 ? 2 * nwarps * NT * 512 : 0));
     int* const warp_sum = lists;                     // kSmallWarps
-    int* const cum = lists + kSmallWarps, *const beg_l = cum + args.groups, *const exp_l = beg_l + args.groups;
+    int* const cum = lists + kSmallWarps;            // per group: tiles up to its end, first row, expert
 
     int ntiles;
-    if (args.experts != nullptr) ntiles = small_scan_groups(args, kTok, cum, beg_l, exp_l, warp_sum);
+    if (args.experts != nullptr) ntiles = small_scan_groups(args, kTok, cum, cum + args.groups, cum + 2 * args.groups, warp_sum);
     else ntiles = (args.rows + kTok - 1) / kTok;
     if (args.tile_count != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *args.tile_count = ntiles;
-    auto tile_of = [&](int tile) -> SmallTile {
-        SmallTile r;
-        if (args.experts == nullptr) {
-            r.expert = 0;
-            r.row0 = tile * kTok;
-            r.ntok = min(kTok, args.rows - r.row0);
-            return r;
-        }
-        int lo = 0, hi = args.groups - 1;   // first group whose cumulative count exceeds the tile
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (cum[mid] > tile) hi = mid; else lo = mid + 1;
-        }
-        const int first = lo > 0 ? cum[lo - 1] : 0;
-        r.expert = exp_l[lo];
-        r.row0 = beg_l[lo] + (tile - first) * kTok;
-        r.ntok = min(kTok, args.offsets[lo] - r.row0);
-        return r;
-    };
+    auto tile_of = [&](int tile) { return small_tile_at(args, kTok, cum, tile); };
 
-    // this CTA's range of units; a unit's coordinates advance by carries, without divisions
-    const int rtg = (N + 16 * rw - 1) / (16 * rw);          // row-tile groups of a weight set
-    const long long units = static_cast<long long>(ntiles) * rtg * args.nsets;
-    const int lo = static_cast<int>(units * blockIdx.x / gridDim.x), hi = static_cast<int>(units * (blockIdx.x + 1) / gridDim.x);
-    struct Unit {
-        int u, tile, set, rg;
-    };
-    Unit first;
-    first.u = lo;
-    first.tile = lo / (rtg * args.nsets);
-    first.set = (lo - first.tile * rtg * args.nsets) / rtg;
-    first.rg = lo - (first.tile * args.nsets + first.set) * rtg;
-    auto advance = [&](Unit& w) {
-        ++w.u;
-        if (++w.rg == rtg) {
-            w.rg = 0;
-            if (++w.set == args.nsets) { w.set = 0; ++w.tile; }
-        }
-    };
+    const SmallWalk walk(args, ntiles);
+    const int hi = walk.hi;
+    using Unit = SmallWalk::Unit;
+    auto advance = [&](Unit& w) { walk.advance(args, w); };
 
     if (Sf::kGridBytes) {
         for (int i = threadIdx.x; i < 1024; i += blockDim.x) reinterpret_cast<uint64_t*>(smem + (grid_s - frag_s))[i] = args.iq2s_grid[i];
@@ -518,7 +637,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
         dst_of[i] = my_ring + r * Sf::kPitch + o;
     }
     const bool rows_aligned = Fmt::kAligned || (row_bytes & 15) == 0;   // all rows of a tile are misaligned alike
-    Unit pu = first;
+    Unit pu = walk.first(args);
     int pkb = ks, p_expert = -1, p_tile = -1;
     bool p_new = true, p_plain = false;
     const uint8_t* p_base = nullptr;   // 16-byte aligned address at or below the unit's first row
@@ -565,7 +684,8 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
     uint32_t slot = 0, parity = 0;
     int cur_tile = -1, turn = 0;
     SmallTile ct = {0, 0, 0};
-    for (Unit un = first; un.u < hi; advance(un)) {
+    bool odd = false;   // this thread has stored a result that is not finite
+    for (Unit un = walk.first(args); un.u < hi; advance(un)) {
         if (un.tile != cur_tile) {
             // ---- x of the token tile as mma fragments
             if (cur_tile >= 0) __syncthreads();
@@ -669,11 +789,13 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
                     __nv_bfloat16* dst = args.out_rows != nullptr ? args.out_rows[r] : args.out[un.set] + static_cast<long long>(r) * N;
                     if (dst != nullptr && row0 + g < N) dst[row0 + g] = __float2bfloat16(v[j]);
                     if (dst != nullptr && row0 + g + 8 < N) dst[row0 + g + 8] = __float2bfloat16(v[2 + j]);
+                    odd |= not_finite(v[j]) || not_finite(v[2 + j]);   // (a row past the last repeats it)
                 }
             }
         }
     }
     cp_async_wait<0>();
+    if (__any_sync(0xFFFFFFFFu, odd)) small_redo<QT, NT>(args, ntiles, cum, my_ring, grid_s);
 }
 
 }  // namespace tgo
