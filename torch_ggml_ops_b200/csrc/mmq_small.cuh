@@ -548,9 +548,9 @@ __device__ __forceinline__ void small_direct(const uint8_t* wgt, long long wgt_b
 __device__ __forceinline__ bool not_finite(float v) { return (__float_as_uint(v) & 0x7F800000u) == 0x7F800000u; }
 
 // After the kernel's walk: every thread looks again at the results that it stored and replaces those
-// that are not finite.  A function of its own, so that the kernel keeps no register for it.
+// that are not finite.
 template <int QT, int NT>
-__device__ __noinline__ void small_redo(const SmallArgs& args, int ntiles, const int* cum, uint32_t my_ring, uint32_t grid_s) {
+__device__ __forceinline__ void small_redo(const SmallArgs& args, int ntiles, const int* cum, uint32_t my_ring, uint32_t grid_s) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int kw = args.kw, rw = args.rw, rwi = warp / kw, ks = warp - rwi * kw;
     const int N = args.out_features, K = args.in_features;
@@ -588,6 +588,13 @@ __device__ __noinline__ void small_redo(const SmallArgs& args, int ntiles, const
     }
 }
 
+// the same as a call, for the kernels that have no register to spare (us inlined / called: 600 tokens, Q3_K
+// experts, 24 tokens per tile 311.6 / 308.8; 16 tokens, IQ2_S experts, 8 per tile 101.7 / 103.7)
+template <int QT, int NT>
+__device__ __noinline__ void small_redo_call(const SmallArgs& args, int ntiles, const int* cum, uint32_t my_ring, uint32_t grid_s) {
+    small_redo<QT, NT>(args, ntiles, cum, my_ring, grid_s);
+}
+
 template <int QT, int NT>
 __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __grid_constant__ SmallArgs args) {
     using Fmt = BlockFmt<QT>;
@@ -619,6 +626,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
     const SmallWalk walk(args, ntiles);
     const int hi = walk.hi;
     using Unit = SmallWalk::Unit;
+    const Unit first = walk.first(args);
     auto advance = [&](Unit& w) { walk.advance(args, w); };
 
     if (Sf::kGridBytes) {
@@ -637,7 +645,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
         dst_of[i] = my_ring + r * Sf::kPitch + o;
     }
     const bool rows_aligned = Fmt::kAligned || (row_bytes & 15) == 0;   // all rows of a tile are misaligned alike
-    Unit pu = walk.first(args);
+    Unit pu = first;
     int pkb = ks, p_expert = -1, p_tile = -1;
     bool p_new = true, p_plain = false;
     const uint8_t* p_base = nullptr;   // 16-byte aligned address at or below the unit's first row
@@ -685,7 +693,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
     int cur_tile = -1, turn = 0;
     SmallTile ct = {0, 0, 0};
     bool odd = false;   // this thread has stored a result that is not finite
-    for (Unit un = walk.first(args); un.u < hi; advance(un)) {
+    for (Unit un = first; un.u < hi; advance(un)) {
         if (un.tile != cur_tile) {
             // ---- x of the token tile as mma fragments
             if (cur_tile >= 0) __syncthreads();
@@ -795,7 +803,10 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
         }
     }
     cp_async_wait<0>();
-    if (__any_sync(0xFFFFFFFFu, odd)) small_redo<QT, NT>(args, ntiles, cum, my_ring, grid_s);
+    if (__any_sync(0xFFFFFFFFu, odd)) {
+        if constexpr (NT <= 2) small_redo<QT, NT>(args, ntiles, cum, my_ring, grid_s);
+        else small_redo_call<QT, NT>(args, ntiles, cum, my_ring, grid_s);
+    }
 }
 
 }  // namespace tgo
