@@ -470,9 +470,17 @@ struct SmallWalk {
     int rtg, lo, hi;
     __device__ __forceinline__ SmallWalk(const SmallArgs& a, int ntiles) {
         rtg = (a.out_features + 16 * a.rw - 1) / (16 * a.rw);   // row-tile groups of a weight set
-        const long long units = static_cast<long long>(ntiles) * rtg * a.nsets;
-        lo = static_cast<int>(units * blockIdx.x / gridDim.x);
-        hi = static_cast<int>(units * (blockIdx.x + 1) / gridDim.x);
+        // = units * b / ctas.  The host has checked that an int holds the units; a dense call's CTA often has one
+        // unit, and two 64-bit divisions before its first load are 0.4 us of 8.7 (grouped: measured no gain)
+        const int units = ntiles * rtg * a.nsets, ctas = gridDim.x, b = blockIdx.x;
+        if (a.experts == nullptr) {
+            const int each = units / ctas, more = units - each * ctas;
+            lo = each * b + more * b / ctas;
+            hi = each * (b + 1) + more * (b + 1) / ctas;
+        } else {
+            lo = static_cast<int>(static_cast<long long>(units) * b / ctas);
+            hi = static_cast<int>(static_cast<long long>(units) * (b + 1) / ctas);
+        }
     }
     __device__ __forceinline__ Unit first(const SmallArgs& a) const {
         Unit w;
