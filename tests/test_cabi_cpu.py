@@ -123,3 +123,31 @@ def test_product_never_imports_the_oracle():
     pkg = ROOT / "torch_ggml_ops_b200"
     for path in list(pkg.rglob("*.py")) + list(pkg.rglob("*.cu*")) + list(pkg.rglob("*.cpp")) + list(pkg.rglob("*.h")):
         assert "oracle" not in path.read_text().lower(), path
+
+
+def test_combine_rows_looks_at_the_output_it_is_given(monkeypatch):
+    """The kernel is given an address and the row count; an output that does not hold them is refused before."""
+    import torch
+    from torch_ggml_ops_b200 import native
+
+    seen = []
+
+    class Library:
+        def tgo_combine_rows(self, rows, pair_to_sorted, weights, out, tokens, top_k, width, stream):
+            seen.append((tokens, top_k, width))
+            return 0
+
+    monkeypatch.setattr(native, "lib", Library)
+    monkeypatch.setattr(native, "_stream", lambda s: None)
+    rows, index = torch.zeros(6, 16, dtype=torch.bfloat16), torch.zeros(12, dtype=torch.int32)
+    bf = torch.bfloat16
+    for bad in (torch.empty(5, 16, dtype=bf), torch.empty(4, 8, dtype=bf), torch.empty(4, 16), torch.empty(64, dtype=bf),
+                torch.empty(16, 4, dtype=bf).t(), torch.empty(4, 16, dtype=bf, device="meta")):
+        with pytest.raises(ValueError, match="out must be"):
+            native.combine_rows(rows, index, 3, out=bad)
+    assert not seen
+    for n in (4, 2):
+        out = torch.empty(n, 16, dtype=bf)
+        assert native.combine_rows(rows, index, 3, out=out) is out
+    assert native.combine_rows(rows, index, 3).shape == (4, 16)
+    assert seen == [(4, 3, 16), (2, 3, 16), (4, 3, 16)]

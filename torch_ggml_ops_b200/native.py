@@ -248,6 +248,10 @@ def combine_rows(rows, pair_to_sorted, top_k, weights=None, stream=None, out=Non
     tokens = pair_to_sorted.numel() // top_k
     if out is None:
         out = torch.empty((tokens, rows.shape[1]), dtype=rows.dtype, device=rows.device)
+    if out.dim() != 2 or out.shape[0] > tokens or out.shape[1] != rows.shape[1] or out.dtype != rows.dtype or out.device != rows.device \
+            or not out.is_contiguous():
+        raise ValueError(f"out must be a contiguous {rows.dtype} tensor of at most {tokens} rows of {rows.shape[1]} on {rows.device}")
+    tokens = out.shape[0]   # a shorter one takes the first tokens
     check(lib().tgo_combine_rows(_ptr(rows), _ptr(pair_to_sorted), _ptr(weights), _ptr(out), tokens, top_k,
                                  rows.shape[1], _stream(stream)), "tgo_combine_rows")
     return out
