@@ -181,3 +181,72 @@ def test_single_process_wrapper(cuda):
     assert ref.rel_frobenius(dx.float().cpu(), want_dx) < CHAIN_TOL
     with pytest.raises(ValueError, match="top_k"):
         mlp.plan(to_dev(torch.from_numpy(ids[:, :1].copy())))
+
+
+def _one_rank(E, H, F, tokens, top_k, cap, tokens_per_rank=None):
+    from torch_ggml_ops_b200.moe_parallel import PeerMoEMLP
+
+    qt_gu, qt_d = ref.Q5_K, ref.Q6_K
+    w = blocks.expert_weights(qt_gu, E, F, H, 3), blocks.expert_weights(qt_gu, E, F, H, 4), blocks.expert_weights(qt_d, E, H, F, 5)
+    W = {k: torch.from_numpy(ref.expert_weights_fp32(a, qt, n, kk))
+         for k, a, qt, n, kk in zip("gud", w, (qt_gu, qt_gu, qt_d), (F, F, H), (H, H, F))}
+    mlp = PeerMoEMLP(*map(to_dev, w), qt_gu, qt_d, E, H, F, capacity_rows=cap, tokens_per_rank=tokens_per_rank or tokens, top_k=top_k)
+    return mlp, W
+
+
+def test_one_rank_phases_by_themselves(cuda):
+    """The phases of ``mlp.r`` after ``mlp.plan`` on one GPU, in an order only separate buffers allow, give what
+    ``forward`` and ``grad_input`` give; so do those with an output of the caller's, which may be shorter."""
+    E, H, F, tokens, top_k = 8, 256, 256, 50, 2
+    mlp, _ = _one_rank(E, H, F, tokens, top_k, tokens * top_k, tokens_per_rank=64)
+    ids = torch.from_numpy(blocks.topk_routing(tokens, E, top_k, seed=2)).clone()
+    ids[3, 1], ids[4] = E, -1   # no such expert: dropped pairs, a token without any
+    gw = to_dev(torch.rand(tokens, top_k))
+    x, dy = (to_dev(blocks.gaussian_bf16((tokens, H), s)) for s in (5, 6))
+    for _ in range(2):
+        mlp.plan(to_dev(ids), gw)
+        y, dx = mlp.forward(x), mlp.grad_input(dy)
+        r = mlp.r
+        r.fwd_send(x)
+        r.bwd_send(dy)
+        r.fwd_compute()
+        r.bwd_compute()
+        assert torch.equal(r.fwd_recv(), y) and torch.equal(r.bwd_recv(), dx)
+        assert not y[4].any() and not dx[4].any()
+    mlp.plan(to_dev(ids))   # without weights, and a phase before anything else of the plan
+    mlp.r.fwd_send(x)
+    mlp.r.fwd_compute()
+    out = torch.full((tokens + 1, H), 7.0, dtype=torch.bfloat16, device="cuda")
+    y = mlp.forward(x, out=out[:tokens])
+    assert y.data_ptr() == out.data_ptr() and torch.equal(mlp.r.fwd_recv(), y) and bool((out[tokens] == 7.0).all())
+    short = torch.full((tokens, H), 7.0, dtype=torch.bfloat16, device="cuda")
+    mlp.grad_input(dy, out=short[:20])
+    assert torch.equal(short[:20], mlp.grad_input(dy)[:20]) and bool((short[20:] == 7.0).all())
+    for bad in (out, torch.empty(tokens, H, device="cuda"), out[:tokens, : H // 2]):
+        with pytest.raises(ValueError, match="out must be"):
+            mlp.forward(x, out=bad)
+
+
+def test_one_rank_overflow(cuda):
+    """Pairs beyond capacity_rows are dropped from the last experts on and reported; the rest is unharmed, and a
+    plan that fits clears the report."""
+    E, H, F, tokens, top_k, cap = 8, 256, 256, 64, 2, 100
+    mlp, W = _one_rank(E, H, F, tokens, top_k, cap)
+    ids = blocks.topk_routing(tokens, E, top_k, seed=2)
+    x, dy = blocks.gaussian_bf16((tokens, H), 5), blocks.gaussian_bf16((tokens, H), 6)
+    mlp.plan(to_dev(torch.from_numpy(ids)))
+    y, dx = mlp.forward(to_dev(x)), mlp.grad_input(to_dev(dy))
+    with pytest.raises(RuntimeError, match="capacity_rows"):
+        mlp.check_overflow()
+    perm, _, _ = blocks.sort_by_expert(ids, E)
+    kept = np.zeros(tokens * top_k, dtype=np.float32)
+    kept[perm[:cap]] = 1.0   # a dropped pair counts as one of weight zero
+    want_y, want_dx = _oracle(W, ids, kept.reshape(tokens, top_k), x, dy)
+    assert ref.rel_frobenius(y.float().cpu(), want_y) < CHAIN_TOL
+    assert ref.rel_frobenius(dx.float().cpu(), want_dx) < CHAIN_TOL
+    few = np.where(np.arange(tokens)[:, None] < 40, ids, -1)
+    mlp.plan(to_dev(torch.from_numpy(few)))
+    mlp.check_overflow()
+    want_y, _ = _oracle(W, ids[:40], None, x[:40], dy[:40])
+    got = mlp.forward(to_dev(x)).float().cpu()
+    assert ref.rel_frobenius(got[:40], want_y) < CHAIN_TOL and not got[40:].any()

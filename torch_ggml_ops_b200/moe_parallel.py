@@ -142,6 +142,16 @@ class MoEMLPRank:
             raise ValueError(f"expected a contiguous torch.bfloat16 tensor of shape {(self.plan['tokens'], self.H)}")
         native.scatter_tokens(tokens, self.plan["pair_row"], self.top_k, self.rows_a)
 
+    def _dst_rank(self) -> torch.Tensor:
+        """The owners of the plan's pairs.  A one-rank plan has none until a phase below is called by itself:
+        the phases work on the exchange buffers, whose maps are then written."""
+        p = self.plan
+        if "dst_rank" not in p:
+            p["dst_rank"] = torch.where(p["pair_row"] >= 0, 0, -1).to(torch.int32)
+            native.ep_token_maps(p["dst_rank"], p["pair_row"], p["tokens"], self.top_k, self.rank, self.tpr, self.peers["row_slot"],
+                                 self.peers["slot_rows"])
+        return p["dst_rank"]
+
     def local_forward(self, x_tokens: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         self._local_in(x_tokens)
         self._experts_forward()
@@ -160,10 +170,11 @@ class MoEMLPRank:
 
     # ------------------------------------------------------------------ forward
     def fwd_send(self, x_tokens: torch.Tensor) -> None:
-        native.ep_dispatch_tokens(x_tokens, self.plan["dst_rank"], self.top_k, self.rank, self.tpr, self.peers["tok_in"])
+        native.ep_dispatch_tokens(x_tokens, self._dst_rank(), self.top_k, self.rank, self.tpr, self.peers["tok_in"])
 
     def fwd_compute(self) -> None:
         """After every rank's ``fwd_send``: this rank's experts, from token rows to partial sums."""
+        self._dst_rank()
         native.ep_expand(self.buf["tok_in"], self.buf["row_slot"], self.plan["n_rows"], self.rows_a)
         self._experts_forward()
         native.ep_reduce(self.rows_b, self.buf["slot_rows"], self.top_k, self.buf["y_part"])
@@ -181,14 +192,15 @@ class MoEMLPRank:
     def fwd_recv(self, out: torch.Tensor | None = None) -> torch.Tensor:
         """After every rank's ``fwd_compute``: [tokens, hidden] = sum of the owners' partial sums."""
         y = out if out is not None else torch.empty(self.plan["tokens"], self.H, dtype=torch.bfloat16, device=self.device)
-        native.ep_pull_tokens(self.peers["y_part"], self.plan["dst_rank"], self.top_k, self.rank, self.tpr, y)
+        native.ep_pull_tokens(self.peers["y_part"], self._dst_rank(), self.top_k, self.rank, self.tpr, y)
         return y
 
     # ------------------------------------------------------------------ input gradient
     def bwd_send(self, dy_tokens: torch.Tensor) -> None:
-        native.ep_dispatch_tokens(dy_tokens, self.plan["dst_rank"], self.top_k, self.rank, self.tpr, self.peers["dy_in"])
+        native.ep_dispatch_tokens(dy_tokens, self._dst_rank(), self.top_k, self.rank, self.tpr, self.peers["dy_in"])
 
     def bwd_compute(self) -> None:
+        self._dst_rank()
         native.ep_expand(self.buf["dy_in"], self.buf["row_slot"], self.plan["n_rows"], self.rows_a)
         self._experts_backward()
         native.ep_reduce(self.rows_b, self.buf["slot_rows"], self.top_k, self.buf["dx_part"])
@@ -205,7 +217,7 @@ class MoEMLPRank:
 
     def bwd_recv(self, out: torch.Tensor | None = None) -> torch.Tensor:
         dx = out if out is not None else torch.empty(self.plan["tokens"], self.H, dtype=torch.bfloat16, device=self.device)
-        native.ep_pull_tokens(self.peers["dx_part"], self.plan["dst_rank"], self.top_k, self.rank, self.tpr, dx)
+        native.ep_pull_tokens(self.peers["dx_part"], self._dst_rank(), self.top_k, self.rank, self.tpr, dx)
         return dx
 
 
