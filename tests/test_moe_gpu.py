@@ -250,3 +250,18 @@ def test_one_rank_overflow(cuda):
     want_y, _ = _oracle(W, ids[:40], None, x[:40], dy[:40])
     got = mlp.forward(to_dev(x)).float().cpu()
     assert ref.rel_frobenius(got[:40], want_y) < CHAIN_TOL and not got[40:].any()
+
+
+def test_one_rank_layer_holds_no_exchange_buffers(cuda):
+    from torch_ggml_ops_b200.moe_parallel import EXCHANGE_BUFFERS
+
+    E, H, F, tokens, top_k = 8, 256, 256, 64, 2
+    mlp, _ = _one_rank(E, H, F, tokens, top_k, tokens * top_k)
+    mlp.plan(to_dev(torch.from_numpy(blocks.topk_routing(tokens, E, top_k, seed=2))))
+    x = to_dev(blocks.gaussian_bf16((tokens, H), 5))
+    y = mlp.forward(x)
+    mlp.grad_input(x)
+    assert not set(EXCHANGE_BUFFERS) & set(mlp.r.buf)
+    mlp.r.fwd_send(x)   # a phase by itself brings them
+    mlp.r.fwd_compute()
+    assert set(EXCHANGE_BUFFERS) <= set(mlp.r.buf) and torch.equal(mlp.r.fwd_recv(), y)

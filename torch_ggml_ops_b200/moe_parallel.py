@@ -31,17 +31,20 @@ import torch.distributed as dist
 
 from . import native
 
-PEER_BUFFERS = ("tok_in", "y_part", "dy_in", "dx_part", "row_slot", "slot_rows", "row_weight", "flags", "counts_tab")
+EXCHANGE_BUFFERS = ("tok_in", "y_part", "dy_in", "dx_part", "row_slot", "slot_rows")
+PEER_BUFFERS = (*EXCHANGE_BUFFERS, "row_weight", "flags", "counts_tab")
 
 
 class MoEMLPRank:
     """One rank of the expert-parallel MLP.  ``w_gate`` / ``w_up``: [E / world, ffn, row bytes] of
     quant type ``qt_gate_up`` (in_features = hidden); ``w_down``: [E / world, hidden, row bytes] of
     ``qt_down`` (in_features = ffn).  ``alloc(name, rows, cols, dtype)`` supplies the buffers the
-    peers address (names in ``PEER_BUFFERS``); ``connect`` then receives every rank's pointers."""
+    peers address (names in ``PEER_BUFFERS``); ``connect`` then receives every rank's pointers.
+    ``lazy_exchange`` (one rank, whose layer needs none of them): the buffers of the token exchange are
+    allocated when a phase is first called by itself."""
 
     def __init__(self, rank, world, w_gate, w_up, w_down, qt_gate_up, qt_down, num_experts, hidden, ffn,
-                 capacity_rows, tokens_per_rank, top_k, alloc=None):
+                 capacity_rows, tokens_per_rank, top_k, alloc=None, lazy_exchange=False):
         if num_experts % world:
             raise ValueError(f"{num_experts} experts do not divide over {world} ranks")
         self.rank, self.world, self.E, self.EL = int(rank), int(world), int(num_experts), num_experts // world
@@ -63,9 +66,9 @@ class MoEMLPRank:
                   "row_slot": (self.cap, 1, i32), "slot_rows": (self.slots, self.top_k, i32),
                   "row_weight": (self.cap, 1, torch.float32),
                   "flags": (1, max(self.world, 2), i32), "counts_tab": (self.world, self.E, i32)}
-        self.buf = {name: alloc(name, *shapes[name]) for name in PEER_BUFFERS}
-        self.buf["slot_rows"].fill_(-1)   # a slot nobody has announced names no row
-        self.buf["row_slot"].fill_(-1)    # a row nobody has announced names no slot
+        self._alloc, self._shapes = alloc, shapes
+        self.buf = {}
+        self._allocate([name for name in PEER_BUFFERS if not (lazy_exchange and name in EXCHANGE_BUFFERS)])
         self.buf["row_weight"].fill_(1.0)
         self.buf["flags"].zero_()         # rank barrier epochs start from zero
         # expert-major rows of this rank only; the wide buffers serve forward and backward in turn
@@ -80,6 +83,12 @@ class MoEMLPRank:
         self.peers = None
         self._route = None
         self.plan = None
+
+    def _allocate(self, names) -> None:
+        for name in names:
+            self.buf[name] = self._alloc(name, *self._shapes[name])
+            if name in ("slot_rows", "row_slot"):
+                self.buf[name].fill_(-1)   # a slot (row) nobody has announced names no row (slot)
 
     def connect(self, peers: dict) -> None:
         """``peers[name][r]`` = device address of rank r's buffer ``name``."""
@@ -147,6 +156,9 @@ class MoEMLPRank:
         the phases work on the exchange buffers, whose maps are then written."""
         p = self.plan
         if "dst_rank" not in p:
+            missing = [name for name in EXCHANGE_BUFFERS if name not in self.buf]
+            self._allocate(missing)
+            self.peers.update({name: [self.buf[name].data_ptr()] for name in missing})
             p["dst_rank"] = torch.where(p["pair_row"] >= 0, 0, -1).to(torch.int32)
             native.ep_token_maps(p["dst_rank"], p["pair_row"], p["tokens"], self.top_k, self.rank, self.tpr, self.peers["row_slot"],
                                  self.peers["slot_rows"])
@@ -253,8 +265,8 @@ class PeerMoEMLP:
         else:
             alloc, ptrs = None, None
         self.r = MoEMLPRank(rank, self.world, w_gate, w_up, w_down, qt_gate_up, qt_down, num_experts, hidden, ffn,
-                            capacity_rows, tokens_per_rank, top_k, alloc=alloc)
-        self.r.connect(ptrs if ptrs is not None else {k: [self.r.buf[k].data_ptr()] for k in PEER_BUFFERS})
+                            capacity_rows, tokens_per_rank, top_k, alloc=alloc, lazy_exchange=self.world == 1)
+        self.r.connect(ptrs if ptrs is not None else {k: [b.data_ptr()] for k, b in self.r.buf.items()})
         self._token = torch.zeros(1, dtype=torch.int32, device=dev)
         self._counts_all = torch.empty(self.world, num_experts, dtype=torch.int32, device=dev)
         if self.world > 1:
