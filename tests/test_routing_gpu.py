@@ -24,6 +24,23 @@ def test_route_sort_is_a_stable_sort_with_cumulative_offsets(cuda, tokens, exper
     assert np.array_equal(p2s.cpu().numpy(), inv.astype(np.int32))
 
 
+# one to eight rounds per block, the last block and its last round part empty; some ids name no expert
+@pytest.mark.parametrize("pairs", [64511, 64513, 72009, 179201, 560001, 1630001])
+def test_route_sort_of_many_pairs(cuda, pairs):
+    from torch_ggml_ops_b200 import native
+
+    experts = 300
+    ids = np.random.default_rng(pairs).integers(-1, experts + 1, size=pairs).astype(np.int32)
+    s2p, p2s, dei, deo = native.route_sort(to_dev(ids), experts)
+    valid = np.flatnonzero((ids >= 0) & (ids < experts))
+    perm = valid[np.argsort(ids[valid], kind="stable")]
+    assert np.array_equal(deo.cpu().numpy(), np.cumsum(np.bincount(ids[valid], minlength=experts)))
+    assert np.array_equal(s2p.cpu().numpy()[: perm.size], perm)
+    inv = np.full(pairs, -1, dtype=np.int32)
+    inv[perm] = np.arange(perm.size)
+    assert np.array_equal(p2s.cpu().numpy(), inv)
+
+
 def test_out_of_range_expert_ids_are_dropped(cuda):
     from torch_ggml_ops_b200 import native
 

@@ -19,9 +19,18 @@ namespace tgo {
 int route_fail(int code, const char* msg);  // defined in tgo_api.cu (sets the thread's error text)
 
 constexpr int kRouteBlock = 256;   // threads of a block; each takes one routed pair per round
-// Rounds per block.  The scan reads one counter per (block, expert) in a single block: with 524288
-// pairs and one round it took 79 us, with eight 10 us.  Few pairs stay spread over the SMs.
-static int route_rounds(int64_t n_pairs) { return n_pairs >= 65536 ? 8 : 1; }
+// Rounds per block.  The scan reads one counter per (block, expert) in a single block, some 0.04 us for
+// every further block; a round, in which the warps of a block take turns, costs all blocks some 4 us: the
+// sum is least at sqrt(blocks / 111) rounds.  us of a sort by 256 experts with 1 / 2 / 3 / 4 / 6 / 8 rounds:
+//      32768 pairs  12.9  14.4  18.3  20.7  28.2  34.4       262144 pairs  42.8  30.1  28.8  29.3  35.2  38.4
+//      65536        17.3  16.6  19.5  21.8  29.3  35.3       524288        81.9  48.5  41.8  38.4  41.1  44.3
+//     131072        25.6  21.3  23.8  24.0  30.5  36.5      1048576       159.3  93.2  78.1  59.1  55.8  55.7
+static int route_rounds(int64_t n_pairs) {
+    const int64_t blocks = (n_pairs + kRouteBlock - 1) / kRouteBlock;
+    int r = 1;
+    while (r < 8 && (2 * r + 1) * (2 * r + 1) * 28 <= blocks) ++r;   // the nearest whole number
+    return r;
+}
 constexpr int kRouteMaxExperts = 4096;
 
 // Pass 1: per-block histogram of expert ids -> block_counts[block][expert].
