@@ -750,10 +750,10 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) tot[nt][0] = tot[nt][1] = tot[nt][2] = tot[nt][3] = 0.f;
         const int row0 = (un.rg * rw + rwi) * 16;
-        int at0 = 0, at1 = 0;   // misalignment of this thread's two rows, before the block's offset
+        uint32_t at0 = 0, at1 = 0;   // misalignment of this thread's two rows, before the block's offset
         if (!Fmt::kAligned) {
             const int row = min(row0, N - 1), last = N - 1 - row;
-            const int first_at = (ct.expert * N + row) * row_bytes;   // only the low bits matter
+            const uint32_t first_at = (static_cast<uint32_t>(ct.expert) * N + row) * row_bytes;   // only the low bits matter
             at0 = first_at + min(g, last) * row_bytes;
             at1 = first_at + min(g + 8, last) * row_bytes;
         }
