@@ -1,5 +1,5 @@
-"""Few tokens per weight row (dense calls of at most 24 rows, sparsely hit experts) take a kernel of
-their own: the edges of its row, token and reduction tiles, its grouped work list and its multi-weight
+"""Few tokens per weight row (dense calls of at most 24 rows whose fragments fit in shared memory, sparsely
+hit experts) take a kernel of their own: the edges of its row, token and reduction tiles, its grouped work list and its multi-weight
 launch, against the fp32 oracle."""
 import numpy as np
 import pytest
@@ -96,6 +96,28 @@ def test_infinite_and_huge_values(cuda, name, qt, M, N, K):
     assert torch.equal(torch.isnan(z[:, 5]), torch.isnan(wide[:, 5])) and torch.equal(torch.nan_to_num(z[:, 5]), torch.nan_to_num(wide[:, 5]))
     keep = torch.arange(N) != 5
     assert torch.equal(z[:, keep], plain[:, keep])
+
+
+@pytest.mark.parametrize("name,qt", ALL_TYPES)
+@pytest.mark.parametrize("M,K,few", [(8, 4096, True), (9, 4096, True), (16, 4096, True), (25, 4096, False), (16, 7168, False),
+                                     (8, 8192, True), (1, 16384, False)])
+def test_shared_memory_limits(cuda, name, qt, M, K, few):
+    """Rows x in_features whose fragments leave room for the slices only if there are fewer of them, or for none:
+    the few-token kernel (which does not round the weights to bf16: a smaller error) or the tile GEMM."""
+    import torch_ggml_ops_b200 as tgo
+
+    N = 40
+    w, W, Wb = dense_case(qt, N, K, 3 + qt)
+    x = blocks.gaussian_bf16((M, K), M)
+    ws = [to_dev(w), to_dev(dense_case(qt, N, K, 4 + qt)[0])]
+    y = tgo.mmq(to_dev(x), ws[0], qt, N)
+    assert ref.rel_frobenius(y.float().cpu(), ref.mmq_forward(x, W)) < 2 * TOL[qt]
+    # rounded weights, exact product: the GEMM's result up to its own rounding to bf16, the other kernel's not
+    rounded = (x.double() @ Wb.double().t()).to(torch.bfloat16)
+    same = float((y.cpu() == rounded).float().mean())
+    if qt != ref.IQ2_S:
+        assert (same < 0.95) == few, same
+    assert torch.equal(tgo.mmq_multi(to_dev(x), ws, qt, N)[0], y)
 
 
 @pytest.mark.parametrize("name,qt", ALL_TYPES)

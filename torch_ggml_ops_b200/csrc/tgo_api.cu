@@ -531,6 +531,12 @@ static int launch_small(int qt, int nt, const SmallArgs& args, int grid, int sme
     }
 }
 
+// Warps that must fit in shared memory beside the fragments of x, which grow with the rows and in_features.
+// us of the GEMM / this kernel by warps, 9 rows, 2048 out-features (8192): 8, Q6_K of 4096 in-features 35.5 / 16.3;
+// 7, Q4_K of 5120 30.7 / 19.6 (31.2 / 30.0); 5, IQ2_S of 12288 91.8 / 30.5 (90.5 / 59.5); 4, Q6_K of 5120
+// 40.0 / 34.5 (41.9 / 54.3); 3, Q4_K of 6144 35.6 / 44.8.  24 rows, 152064 x 4096: 1 (Q6_K) 276 / 1146, 4 (Q4_K)
+// 183 / 326.  So 8 rows take it up to 10240 (Q6_K) .. 12544 (IQ2_S) in-features, 16 to 4864 .. 5888, 24 to 3072 .. 3840.
+constexpr int64_t kSmallLeastWarps = 5;
 constexpr int64_t kSmallRounds = 3;     // row tiles per warp from which on the reduction is not sliced
 // Most rows per group for which the few-token kernel is the faster one.  Its time grows with the
 // tokens (every 8 are one more mma per fragment), the GEMM's hardly does below 256.  Dense: measured
@@ -572,20 +578,27 @@ static bool plan_small(const Problem& p, SmallPlan& s) {
     int64_t kw = (kSmallRounds * warps + set_tiles - 1) / set_tiles;
     if (kw > nkb) kw = nkb;
     if (kw > kSmallWarps) kw = kSmallWarps;
-    const int64_t rounds = (nkb + kw - 1) / kw;
-    s.kw = static_cast<int>((nkb + rounds - 1) / rounds);   // the fewest slices with that many blocks at most
-    int64_t rw = kSmallWarps / s.kw;
-    if (rw > row_tiles / num_sms()) rw = row_tiles / num_sms();
-    if (rw < 1) rw = 1;
     const int lists = p.experts != nullptr ? static_cast<int>(groups) : 0;
-    for (;; --rw) {
-        if (rw < 1) return false;   // the fragments of x alone do not fit
+    auto fits = [&](int64_t rw, int stages) {
         s.rw = static_cast<int>(rw);
-        for (s.stages = 4; s.stages >= 2; --s.stages) {
-            s.smem = small_smem(p.qt, nkb, s.nt, s.kw, s.rw, s.stages, lists);
-            if (s.smem <= kSmallSmemLimit) break;
+        s.stages = stages;
+        s.smem = small_smem(p.qt, nkb, s.nt, s.kw, s.rw, stages, lists);
+        return s.smem <= kSmallSmemLimit;
+    };
+    for (;;) {
+        const int64_t rounds = (nkb + kw - 1) / kw;
+        s.kw = static_cast<int>((nkb + rounds - 1) / rounds);   // the fewest slices with that many blocks at most
+        int64_t rw = kSmallWarps / s.kw;
+        while (rw > 0 && !fits(rw, 2)) --rw;
+        if (rw * s.kw >= kSmallLeastWarps || (rw > 0 && rw == kSmallWarps / s.kw)) {
+            if (rw > row_tiles / num_sms()) rw = row_tiles / num_sms();
+            if (rw < 1) rw = 1;
+            if (!fits(rw, 4) && !fits(rw, 3)) fits(rw, 2);
+            break;
         }
-        if (s.stages >= 2) break;
+        // too few warps for what is left beside the fragments of x: fewer slices, whose partial sums need less
+        kw = s.kw - 1;
+        if (kw < kSmallLeastWarps) return false;
     }
     int per_sm = kSmallWarps / (s.kw * s.rw);                 // 128 registers a thread
     const int fit = kSmallSmemLimit / (s.smem + 1024);
