@@ -4,7 +4,8 @@ Produces, next to this file:
 
 * ``lib/libtgo_mmq.so``  - the C-ABI CUDA library (``include/tgo_mmq.h``), compiled by nvcc for
   ``sm_100a`` only (``-gencode arch=compute_100a,code=sm_100a``);
-* ``_ext.abi3.so``       - autograd formulas and this package's own operators (libtorch's C++ API);
+* ``_ext.abi3.so``       - autograd formulas and this package's own operators (libtorch's C++ API: for
+  the torch release it was built with, and rebuilt for another);
 * ``_C.abi3.so``         - the libtorch stable-ABI module that registers the
   ``torch_ggml_ops::*`` operators over that C ABI (reference build recipe: setup.py:23-44,
   ``-DTORCH_TARGET_VERSION=0x020A000000000000 -DTORCH_STABLE_ONLY``).
@@ -146,7 +147,10 @@ def build_ext(force: bool = False) -> Path:
     import torch
 
     src = CSRC / "torch_ext.cpp"
-    if not force and _newer(EXT_PATH, [src, ROOT / "include" / "tgo_mmq.h", LIB_PATH]):
+    # libtorch's C++ ABI holds for one torch release, so the release is part of what the module is built from
+    built_for = BUILD / "torch_ext.torch_version"
+    if not force and _newer(EXT_PATH, [src, ROOT / "include" / "tgo_mmq.h", LIB_PATH]) and built_for.exists() \
+            and built_for.read_text() == torch.__version__:
         return EXT_PATH
     tdir = Path(torch.__file__).resolve().parent
     cuda = Path(_nvcc()).resolve().parents[1]
@@ -157,6 +161,8 @@ def build_ext(force: bool = False) -> Path:
           *[f"-I{p}" for p in inc], str(src), "-o", str(EXT_PATH),
           f"-L{LIB_DIR}", "-ltgo_mmq", f"-L{tdir / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
           "-Wl,-rpath,$ORIGIN/lib", f"-Wl,-rpath,{tdir / 'lib'}"])
+    BUILD.mkdir(parents=True, exist_ok=True)
+    built_for.write_text(torch.__version__)
     return EXT_PATH
 
 
