@@ -235,17 +235,18 @@ std::vector<Tensor> multi_cuda(const Tensor& x, at::TensorList ws, int64_t qt, i
              "tgo_mmq_fwd_multi");
     return ys;
 }
-std::vector<Tensor> call_multi(const Tensor& x, at::TensorList ws, int64_t qt, int64_t n) {
-    static const auto h = op<std::vector<Tensor>(const Tensor&, at::TensorList, int64_t, int64_t)>("torch_ggml_ops_b200::mmq_multi");
-    return h.call(x, ws, qt, n);
+// its integers may be symbolic in a traced program
+std::vector<Tensor> call_multi(const Tensor& x, at::TensorList ws, c10::SymInt qt, c10::SymInt n) {
+    static const auto h = op<std::vector<Tensor>(const Tensor&, at::TensorList, c10::SymInt, c10::SymInt)>("torch_ggml_ops_b200::mmq_multi");
+    return h.call(x, ws, std::move(qt), std::move(n));
 }
 struct MultiFn : public Function<MultiFn> {
-    static variable_list forward(AutogradContext* ctx, const Tensor& x, std::vector<Tensor> ws, int64_t qt, int64_t n) {
+    static variable_list forward(AutogradContext* ctx, const Tensor& x, std::vector<Tensor> ws, c10::SymInt qt, c10::SymInt n) {
         at::AutoDispatchBelowADInplaceOrView guard;
-        ctx->saved_data["qt"] = qt;
+        ctx->saved_data["qt"] = qt.guard_int(__FILE__, __LINE__);
         ctx->saved_data["k"] = last_size(x, -1);
         ctx->set_materialize_grads(false);
-        variable_list y = call_multi(x, ws, qt, n);
+        variable_list y = call_multi(x, ws, std::move(qt), std::move(n));
         ctx->save_for_backward(std::move(ws));
         return y;
     }
@@ -263,10 +264,10 @@ struct MultiFn : public Function<MultiFn> {
         return {total, Tensor(), Tensor(), Tensor()};
     }
 };
-std::vector<Tensor> multi_autograd(const Tensor& x, at::TensorList ws, int64_t qt, int64_t n) {
-    if (wants_grad(x)) return MultiFn::apply(x, ws.vec(), qt, n);
+std::vector<Tensor> multi_autograd(const Tensor& x, at::TensorList ws, c10::SymInt qt, c10::SymInt n) {
+    if (wants_grad(x)) return MultiFn::apply(x, ws.vec(), std::move(qt), std::move(n));
     at::AutoDispatchBelowADInplaceOrView guard;
-    return call_multi(x, ws, qt, n);
+    return call_multi(x, ws, std::move(qt), std::move(n));
 }
 
 // ------------------------------------------------------------------ swiglu
@@ -466,7 +467,7 @@ TORCH_LIBRARY_IMPL(torch_ggml_ops, Autograd, m) {
 }
 
 TORCH_LIBRARY_FRAGMENT(torch_ggml_ops_b200, m) {
-    m.def("mmq_multi(Tensor input, Tensor[] packed_weights, int quant_type, int out_features) -> Tensor[]");
+    m.def("mmq_multi(Tensor input, Tensor[] packed_weights, SymInt quant_type, SymInt out_features) -> Tensor[]");
     m.def("swiglu(Tensor gate, Tensor up) -> Tensor");
     m.def("swiglu_grad(Tensor grad, Tensor gate, Tensor up) -> (Tensor, Tensor)");
     m.def(
