@@ -29,6 +29,21 @@ def test_dense(cuda, name, qt, M, N, K):
 
 
 @pytest.mark.parametrize("name,qt", ALL_TYPES)
+def test_no_less_exact_than_rounded_weights(cuda, name, qt):
+    """Against 64 bits: at most the error of the exact product with weights rounded to bf16, as the GEMM has
+    them, rounded to bf16 (98304 results: either error is known to a quarter of a percent)."""
+    import torch_ggml_ops_b200 as tgo
+
+    M, N, K = 24, 4096, 1024
+    w, W, Wb = dense_case(qt, N, K, 30 + qt)
+    x = blocks.gaussian_bf16((M, K), M)
+    want = x.double() @ torch.from_numpy(W).double().t()
+    rounded = (x.double() @ Wb.double().t()).to(torch.bfloat16).double()
+    y = tgo.mmq(to_dev(x), to_dev(w), qt, N).double().cpu()
+    assert float((y - want).norm()) < float((rounded - want).norm())
+
+
+@pytest.mark.parametrize("name,qt", ALL_TYPES)
 @pytest.mark.parametrize("N,K", [(72, 2048), (40, 512)])
 @pytest.mark.parametrize("sizes", [[1, 0, 8, 9, 3, 40, 2, 1], [28, 1, 10, 17, 7, 9]])
 def test_grouped_pair_and_invalid_groups(cuda, name, qt, N, K, sizes):
@@ -115,8 +130,7 @@ def test_shared_memory_limits(cuda, name, qt, M, K, few):
     # rounded weights, exact product: the GEMM's result up to its own rounding to bf16, the other kernel's not
     rounded = (x.double() @ Wb.double().t()).to(torch.bfloat16)
     same = float((y.cpu() == rounded).float().mean())
-    if qt != ref.IQ2_S:
-        assert (same < 0.95) == few, same
+    assert (same < 0.95) == few, same
     assert torch.equal(tgo.mmq_multi(to_dev(x), ws, qt, N)[0], y)
 
 
