@@ -104,7 +104,7 @@ int tgo_mmq_dx_ws(const void* dy, const void* packed_weight, void* dx, int64_t r
 /* Several dense projections of the same activations in one call: ys[i] = X * W_i^T for
  * num_weights (1..4) packed weights of the same quant type and shape [out_features, in_features];
  * packed_weights and ys are HOST arrays of device pointers.  Two weight sets share a launch, as the
- * gate/up pair does in tgo_grouped_fwd; every ys[i] is bit-identical to tgo_mmq_fwd on W_i alone.
+ * gate/up pair does in tgo_grouped_fwd (few rows: all of them); every ys[i] is bit-identical to tgo_mmq_fwd on W_i alone.
  * No counterpart in the reference, which lists a dense pair / multi-projection operator as its
  * remaining dense-forward work (docs/mmq_fwd_optimization.md:299-307: there the shared cost is the
  * q8_1 quantisation of the activations, which this library's bf16 path does not have at all). */

@@ -15,7 +15,8 @@
 // [weight row n][64 k] is a K-major operand forward and an MN-major operand backward, so neither
 // direction transposes.  The reduction order of every output element is fixed (ascending
 // reduction index, 16 per UMMA), independent of tiling, which makes grouped == dense and
-// pair == two singles bit-exact.
+// pair == two singles bit-exact among the calls that this kernel takes (forward products of few tokens
+// per weight row go to mmq_small.cuh, which rounds no weight and adds in another order).
 //
 // CG = 2 (the default): two CTAs of a cluster share a token tile and cover 256 weight rows with
 // cta_group::2 UMMAs; each CTA decodes its own 128 rows and stages half of the tokens, the

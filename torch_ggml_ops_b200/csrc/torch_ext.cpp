@@ -66,8 +66,8 @@ Tensor call_pair_dx(const Tensor& d0, const Tensor& d1, const Tensor& w0, const 
 }
 
 bool wants_grad(const Tensor& t) { return at::GradMode::is_enabled() && t.requires_grad(); }
-// A cotangent handed over by autograd may be a view; the operators refuse what is not contiguous
-// or starts inside a storage.
+// A cotangent handed over by autograd may be a transposed view; the operators refuse what is not
+// contiguous.  (One that starts inside a storage stays as it is, and is refused.)
 Tensor plain(const Tensor& g) { return g.contiguous(); }
 
 [[noreturn]] void no_second_order(const char* name) {

@@ -48,8 +48,8 @@ def _(hidden, packed_weight, quant_type, vocab, targets, chunk_rows, grad_scale)
 
 def mmq_multi(input: torch.Tensor, packed_weights, quant_type: int, out_features: int):
     """``[input @ W_i.T for W_i in packed_weights]`` (1 to 4 weights of one quant type and shape
-    [out_features, in_features]) with two weight sets per kernel launch; every result is
-    bit-identical to ``mmq`` on that weight alone."""
+    [out_features, in_features]) with two weight sets per kernel launch (few tokens: all of them); every
+    result is bit-identical to ``mmq`` on that weight alone."""
     return tuple(_ops.mmq_multi.default(input, list(packed_weights), int(quant_type), int(out_features)))
 
 
@@ -77,6 +77,8 @@ def lm_head_loss(hidden: torch.Tensor, packed_weight: torch.Tensor, quant_type: 
     (bf16 logits) -> fp32 log-softmax and loss, cotangent ``(softmax - onehot) * grad_scale`` in
     bf16 over the logits -> input gradient.  Returns ``(loss_sum fp32 scalar tensor, d_hidden bf16
     like hidden)``.
+
+    The loss is differentiable with respect to ``hidden``, once; the returned gradient is not.
 
     The reference's production consumer runs this loop with chunk_rows = 256 for a Q6_K head of
     248320 x 2048 (docs/mmq_bwd_optimization.md:502-524); rows = hidden.numel() / K."""
