@@ -703,7 +703,9 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
     uint32_t slot = 0, parity = 0;
     int cur_tile = -1, turn = 0;
     SmallTile ct = {0, 0, 0};
-    bool odd = false;   // this thread has stored a result that is not finite
+    // stays zero while this thread's results are finite: infinities and NaN times zero are NaN.  (Two
+    // instructions per 8 tokens; tests of each result cost 2-4 % where the reduction has two blocks.)
+    float2 odd = make_float2(0.f, 0.f);
     for (Unit un = first; un.u < hi; advance(un)) {
         if (un.tile != cur_tile) {
             // ---- x of the token tile as mma fragments
@@ -800,6 +802,8 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
                     v[3] += __uint_as_float(p.w);
                 }
             }
+            odd = __ffma2_rn(make_float2(v[0], v[1]), make_float2(0.f, 0.f), odd);
+            odd = __ffma2_rn(make_float2(v[2], v[3]), make_float2(0.f, 0.f), odd);
             const int token = nt * 8 + 2 * t;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -808,13 +812,12 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
                     __nv_bfloat16* dst = args.out_rows != nullptr ? args.out_rows[r] : args.out[un.set] + static_cast<long long>(r) * N;
                     if (dst != nullptr && row0 + g < N) dst[row0 + g] = __float2bfloat16(v[j]);
                     if (dst != nullptr && row0 + g + 8 < N) dst[row0 + g + 8] = __float2bfloat16(v[2 + j]);
-                    odd |= not_finite(v[j]) || not_finite(v[2 + j]);   // (a row past the last repeats it)
                 }
             }
         }
     }
     cp_async_wait<0>();
-    if (__any_sync(0xFFFFFFFFu, odd)) {
+    if (__any_sync(0xFFFFFFFFu, odd.x != 0.f || odd.y != 0.f)) {
         if constexpr (NT <= 2) small_redo<QT, NT>(args, ntiles, cum, my_ring, grid_s);
         else small_redo_call<QT, NT>(args, ntiles, cum, my_ring, grid_s);
     }
