@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 1) mmq_small_kernel(const __
     int cur_tile = -1, turn = 0;
     SmallTile ct = {0, 0, 0};
     // stays zero while this thread's results are finite: infinities and NaN times zero are NaN.  (Two
-    // instructions per 8 tokens; tests of each result cost 2-4 % where the reduction has two blocks.)
+    // instructions per 8 tokens; tests of each result cost 1-4 % where the reduction has two blocks.)
     float2 odd = make_float2(0.f, 0.f);
     for (Unit un = first; un.u < hi; advance(un)) {
         if (un.tile != cur_tile) {

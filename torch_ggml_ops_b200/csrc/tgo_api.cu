@@ -531,12 +531,14 @@ static int launch_small(int qt, int nt, const SmallArgs& args, int grid, int sme
     }
 }
 
-// Warps that must fit in shared memory beside the fragments of x, which grow with the rows and in_features.
-// us of the GEMM / this kernel by warps, 9 rows, 2048 out-features (8192): 8, Q6_K of 4096 in-features 35.5 / 16.3;
-// 7, Q4_K of 5120 30.7 / 19.6 (31.2 / 30.0); 5, IQ2_S of 12288 91.8 / 30.5 (90.5 / 59.5); 4, Q6_K of 5120
-// 40.0 / 34.5 (41.9 / 54.3); 3, Q4_K of 6144 35.6 / 44.8.  24 rows, 152064 x 4096: 1 (Q6_K) 276 / 1146, 4 (Q4_K)
-// 183 / 326.  So 8 rows take it up to 10240 (Q6_K) .. 12544 (IQ2_S) in-features, 16 to 4864 .. 5888, 24 to 3072 .. 3840.
-constexpr int64_t kSmallLeastWarps = 5;
+// Warps that must fit in shared memory beside the fragments of x, which grow with the rows and in_features,
+// by groups of 8 rows.  us of the GEMM / this kernel, 2048 out-features (8192):
+//   8 rows, 5 warps, IQ2_S of 12288 in-features  91.8 / 30.5 (90.5 / 59.5)    3, Q4_K of 12288  65.9 / 49.1 (64.1 / 87.0)
+//   16, 8, Q6_K of 4096  35.5 / 16.4    7, Q4_K of 5120  30.8 / 20.1 (31.2 / 30.0)    4, Q6_K of 5120  40.0 / 34.3 (42.0 / 54.1)
+//   24, 5, IQ2_S of 3840, 9000 out-features  32.8 / 39.8    4, IQ2_S of 4096  33.8 / 29.2 (34.1 / 41.5)
+//   24, 152064 x 4096: 1, Q6_K  276 / 1146    4, Q4_K  183 / 326
+// So 8 rows take it up to 10240 (Q6_K) .. 12544 (IQ2_S) in-features, 16 up to 4096 .. 5376, 24 to some 2560.
+static int64_t small_least_warps(int nt) { return nt == 1 ? 5 : nt == 2 ? 7 : 8; }
 constexpr int64_t kSmallRounds = 3;     // row tiles per warp from which on the reduction is not sliced
 // Most rows per group for which the few-token kernel is the faster one.  Its time grows with the
 // tokens (every 8 are one more mma per fragment), the GEMM's hardly does below 256.  Dense: measured
@@ -590,7 +592,7 @@ static bool plan_small(const Problem& p, SmallPlan& s) {
         s.kw = static_cast<int>((nkb + rounds - 1) / rounds);   // the fewest slices with that many blocks at most
         int64_t rw = kSmallWarps / s.kw;
         while (rw > 0 && !fits(rw, 2)) --rw;
-        if (rw * s.kw >= kSmallLeastWarps || (rw > 0 && rw == kSmallWarps / s.kw)) {
+        if (rw * s.kw >= small_least_warps(s.nt) || (rw > 0 && rw == kSmallWarps / s.kw)) {
             if (rw > row_tiles / num_sms()) rw = row_tiles / num_sms();
             if (rw < 1) rw = 1;
             if (!fits(rw, 4) && !fits(rw, 3)) fits(rw, 2);
@@ -598,7 +600,7 @@ static bool plan_small(const Problem& p, SmallPlan& s) {
         }
         // too few warps for what is left beside the fragments of x: fewer slices, whose partial sums need less
         kw = s.kw - 1;
-        if (kw < kSmallLeastWarps) return false;
+        if (kw < small_least_warps(s.nt)) return false;
     }
     int per_sm = kSmallWarps / (s.kw * s.rw);                 // 128 registers a thread
     const int fit = kSmallSmemLimit / (s.smem + 1024);
